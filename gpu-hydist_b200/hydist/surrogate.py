@@ -45,17 +45,26 @@ def pad16(c):
     return (c + 15) // 16 * 16
 
 
+_bound = None
+
+
 def _bind():
+    global _bound
+    if _bound is not None:
+        return _bound
     lib = hlib.load()
     P, I, L, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
     lib.hyd_conv_forward.restype = I
     lib.hyd_conv_forward.argtypes = [P, I, I, I, I, P, P, I, I, I, I, P, P, I, I, I, P, P]
     lib.hyd_conv_wgrad.restype = I
     lib.hyd_conv_wgrad.argtypes = [P, I, I, I, I, I, P, I, I, I, I, P, P, P]
+    lib.hyd_conv_pack.restype = I
+    lib.hyd_conv_pack.argtypes = [P, I, I, L, L, L, I, I, P, P]
     lib.hyd_bias_grad.restype = I
     lib.hyd_bias_grad.argtypes = [P, L, I, I, P, P]
     lib.hyd_mse_grad.restype = I
     lib.hyd_mse_grad.argtypes = [P, P, P, L, I, I, F, P, P, P]
+    _bound = lib
     return lib
 
 
@@ -79,9 +88,19 @@ def pack_index(ncol, cinp, device):
 
 def pack_weights(w, ncol, cinp):
     """w: FP32 [nout][9][cin] -> the BF16 shared-memory image for ncol output columns and
-    cinp (>= cin) input channels per pixel."""
+    cinp (>= cin) input channels per pixel.  On the device one kernel packs it, whatever the
+    strides of w (the six PyTorch operations below took 32 us there, most of a layer)."""
     import torch
-    nout, _, cin = w.shape
+    nout, taps, cin = w.shape
+    if w.is_cuda and w.dtype == torch.float32 and taps == 9 and w.numel() > 0 and not w.requires_grad and \
+            ncol % 16 == 0 and cinp % 16 == 0 and nout <= ncol <= 256 and cin <= cinp <= 256:
+        img = torch.empty(ncol * 9 * cinp, dtype=torch.bfloat16, device=w.device)
+        with torch.cuda.device(w.device):
+            rc = _bind().hyd_conv_pack(w.data_ptr(), nout, cin, *w.stride(), ncol, cinp, img.data_ptr(),
+                                       torch.cuda.current_stream(w.device).cuda_stream)
+        if rc != 0:
+            raise hlib.HydError("hyd_conv_pack failed (%d)" % rc)
+        return img
     full = torch.zeros((ncol, 9, cinp), dtype=torch.float32, device=w.device)
     full[:nout, :, :cin] = w
     img = torch.empty(ncol * 9 * cinp, dtype=torch.bfloat16, device=w.device)
@@ -183,7 +202,7 @@ class Surrogate:
             if l == 0:
                 break
             # data gradient, fused with the ReLU derivative of this layer's input
-            wt = self.w[l].permute(2, 1, 0).contiguous()  # [cin][9][cout]
+            wt = self.w[l].permute(2, 1, 0)  # [cin][9][cout]
             wpk = pack_weights(wt, pad16(cin), ncol)
             dy = self.conv(dy, B, Ho, Wo, ncol, wpk, None, pad16(cin), cin, ADJOINT[mode], False, Hi, Wi, mask=x)
         return gw, gb

@@ -470,6 +470,9 @@ int hyd_get_sweep_shape(hyd_handle h, int* ctas, int* wide);
  *   (n / 8) 256 + (k / 8) 128 + (n % 8) 16 + (k % 8) 2.  relu: max(0, .); out_f32: FP32
  *   output instead of BF16.  *err is set to 1 if a wait on the tensor cores timed out.
  *   B x Hout x Wout must stay below 2^31 (HYD_EINVAL otherwise).
+ * hyd_conv_pack: that image from FP32 weights, element (n, t, c) at w[n sn + t st + c sc] for
+ *   n < nout, c < cin, zero up to ncol and cinp (multiples of 16, at most 256); strides, so that
+ *   a data gradient's channel-transposed weights are packed from the layer's own.
  * hyd_conv_wgrad: dw[n][t][c] += sum_p dy[p][n] x[map(p,t)][c] (FP32, n < nout), dy with
  *   ncol channels per pixel; map is the layer's forward mapping.
  * hyd_bias_grad: db[n] += sum_p dy[p][n].
@@ -485,6 +488,8 @@ int hyd_get_sweep_shape(hyd_handle h, int* ctas, int* wide);
 int hyd_conv_forward(const void* x, int B, int Hin, int Win, int cin, const void* w_packed, const float* bias,
                      int ncol, int nout, int mode, int relu, const void* mask, void* y, int Hout, int Wout,
                      int out_f32, int* err, void* stream);
+int hyd_conv_pack(const float* w, int nout, int cin, long long sn, long long st, long long sc, int ncol, int cinp,
+                  void* w_packed, void* stream);
 int hyd_conv_wgrad(const void* x, int B, int Hin, int Win, int cin, int mode, const void* dy, int Hout, int Wout,
                    int ncol, int nout, float* dw, int* err, void* stream);
 int hyd_bias_grad(const void* dy, long long npix, int ncol, int nout, float* db, void* stream);

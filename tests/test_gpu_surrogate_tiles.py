@@ -105,3 +105,56 @@ def test_wgrad_tiles(mode, size):
         n = B * (Ho + 3) * (Wo + 3) + 32  # additions of one element, the raster's padding included
         assert bool(((dw.double() - ref).abs() <= n * ULP * mag).all())
     net.check_errors()
+
+
+@pytest.mark.parametrize("npix,ncol,nout,shift", [(1, 48, 48, 0), (33, 16, 3, 0), (70001, 48, 41, 0), (5000, 256, 256, 0),
+                                                  (777, 48, 48, 1), (900, 20, 7, 0), (64, 264, 10, 0)])
+def test_bias_grad_tiles(npix, ncol, nout, shift):
+    """Channel sums over the pixels against 64 bits (npix additions, db added at the end)."""
+    import torch
+    from hydist import surrogate as S
+    g = torch.Generator(device="cuda").manual_seed(npix)
+    net = S.Surrogate()
+    dy = torch.randn(npix * ncol + shift, generator=g, device="cuda").to(torch.bfloat16)[shift:]
+    db0 = torch.randn(nout, generator=g, device="cuda")
+    db = db0.clone()
+    assert net.lib.hyd_bias_grad(dy.data_ptr(), npix, ncol, nout, db.data_ptr(), net._stream()) == 0
+    d = dy.view(npix, ncol)[:, :nout].double()
+    ref, mag = d.sum(0) + db0.double(), d.abs().sum(0) + db0.double().abs()
+    assert bool(((db.double() - ref).abs() <= (npix + 1) * ULP * mag).all())
+
+
+@pytest.mark.parametrize("npix,nc,ncol,weighted,shift", [(1, 3, 16, True, 0), (4099, 3, 16, False, 0), (700, 5, 16, True, 0),
+                                                         (513, 3, 20, True, 0), (300, 4, 8, True, 0), (300, 3, 16, True, 1)])
+def test_mse_grad_tiles(npix, nc, ncol, weighted, shift):
+    """The loss against 64 bits and the gradient as the rounded FP32 expression."""
+    import torch
+    from hydist import surrogate as S
+    g = torch.Generator(device="cuda").manual_seed(npix)
+    net = S.Surrogate()
+    a, b = torch.randn((2, npix, nc), generator=g, device="cuda")
+    w = torch.rand(npix, generator=g, device="cuda") if weighted else None
+    dy = torch.empty(npix * ncol + shift, dtype=torch.bfloat16, device="cuda")[shift:]
+    loss = torch.zeros(1, device="cuda")
+    scale = 0.125
+    assert net.lib.hyd_mse_grad(a.data_ptr(), b.data_ptr(), w.data_ptr() if weighted else None, npix, nc, ncol, scale,
+                                dy.data_ptr(), loss.data_ptr(), net._stream()) == 0
+    wt = w[:, None] if weighted else torch.ones((npix, 1), device="cuda")
+    want = torch.zeros((npix, ncol), device="cuda")
+    want[:, :nc] = 2.0 * wt * (a - b) * scale
+    assert torch.equal(dy.view(npix, ncol), want.to(torch.bfloat16))
+    ref = (wt.double() * (a.double() - b.double()) ** 2).sum() * scale
+    assert abs(float(loss) - float(ref)) <= (npix * nc + 8) * 4 * ULP * float(ref)
+
+
+@pytest.mark.parametrize("nout,cin,ncol,cinp", [(48, 48, 48, 48), (48, 6, 48, 16), (3, 48, 16, 48), (1, 1, 16, 16)])
+def test_pack_matches_the_layout(nout, cin, ncol, cinp):
+    """The packing kernel against the layout's formula (pack_index), for weights as they lie
+    and for a transposed view."""
+    import torch
+    from hydist import surrogate as S
+    w = torch.randn((nout, 9, cin), generator=torch.Generator().manual_seed(1))
+    for v, a, b in ((w, ncol, cinp), (w.permute(2, 1, 0), cinp, ncol)):
+        want = S.pack_weights(v, a, b)  # on the CPU: PyTorch
+        dev = w.cuda() if v is w else w.cuda().permute(2, 1, 0)
+        assert torch.equal(S.pack_weights(dev, a, b).cpu(), want)

@@ -89,7 +89,7 @@ struct HydSim {
     int solver;
     int start_idx, end_idx;
     unsigned* h_status;
-    double* run_part;  // hyd_run's non-finite check: partial sums, allocated at its first use
+    double* run_part;  // the mass-balance kernels' partial sums, allocated at their first use
     // phase timing (instrumentation): bit k set = phase k bracketed by events
     unsigned timing;
     struct Mark {
@@ -354,25 +354,29 @@ int check_device_status(HydSim* s) {
     return HYD_OK;
 }
 
-// mass balance: per-block partial sums, then one block adds them in a fixed order
-__global__ void k_mass_partial(DevGrid g, double* part) {
+// mass balance: per-block partial sums, then one block adds them in a fixed order.  One warp
+// per row, every field of a cell loaded before it is tested (a row takes its passes' memory
+// round trips side by side).  A cell at a time in grid order, its row and column by 64-bit
+// divisions, and one thread adding the partials, took about 200 us on a 1048 x 980 grid.
+__global__ void __launch_bounds__(256) k_mass_partial(DevGrid g, double* part) {
     __shared__ double sh[5][256];
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     double a = 0, b = 0, c = 0, wet = 0, bad = 0;
-    const long long ncell = (long long)(g.N + 3) * (g.M + 3);
-    for (long long q = (long long)blockIdx.x * blockDim.x + tid; q < ncell; q += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(q / (g.M + 3)), j = (int)(q % (g.M + 3));
-        const int gp = i * g.P + j;
-        if (i <= g.N && j <= g.M) {
-            if (!isfinite(g.z[gp]) || !isfinite(g.u[gp]) || !isfinite(g.v[gp]) || !isfinite(g.FS[gp])) bad += 1;
+    for (int i = (blockIdx.x * blockDim.x + tid) >> 5; i <= g.N; i += (gridDim.x * blockDim.x) >> 5) {
+#pragma unroll 4
+        for (int j = lane; j <= g.M; j += 32) {
+            const int gp = i * g.P + j;
+            const double z = g.z[gp], u = g.u[gp], v = g.v[gp], fs = g.FS[gp], H = g.H_moi[gp], dh = g.dH[gp];
+            const int kh = g.khouot[gp];
+            if (!isfinite(z) || !isfinite(u) || !isfinite(v) || !isfinite(fs)) bad += 1;
+            if (i < 2 || j < 2) continue;
+            if (kh == 0) {
+                a += H;
+                b += fs * H;
+                wet += 1;
+            }
+            if (isfinite(dh)) c += dh;
         }
-        if (i < 2 || j < 2 || i > g.N || j > g.M) continue;
-        if (g.khouot[gp] == 0) {
-            a += g.H_moi[gp];
-            b += g.FS[gp] * g.H_moi[gp];
-            wet += 1;
-        }
-        if (isfinite(g.dH[gp])) c += g.dH[gp];
     }
     sh[0][tid] = a;
     sh[1][tid] = b;
@@ -389,12 +393,13 @@ __global__ void k_mass_partial(DevGrid g, double* part) {
         for (int k = 0; k < 5; k++) part[blockIdx.x * 5 + k] = sh[k][0];
 }
 
+// Five warps, one per sum.
 __global__ void k_mass_final(const double* part, int nblocks, double* out) {
-    if (threadIdx.x != 0) return;
-    double acc[5] = {0, 0, 0, 0, 0};
-    for (int b = 0; b < nblocks; b++)
-        for (int k = 0; k < 5; k++) acc[k] += part[b * 5 + k];
-    for (int k = 0; k < 5; k++) out[k] = acc[k];
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double acc = 0;
+    for (int b = lane; b < nblocks; b += 32) acc += part[b * 5 + k];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) out[k] = acc;
 }
 
 // Scratch of hyd_mass_balance_noalloc: up to HYD_MASS_NOALLOC_MAX_BLOCKS blocks of five
@@ -1281,19 +1286,27 @@ int hyd_step(hyd_handle h, int nsteps, int sync, double* t_out) {
     return HYD_OK;
 }
 
+// The mass-balance sums (k_mass_partial) on the handle's stream, waited for; the partial sums in
+// the handle's own buffer, allocated at the first call (an allocation from the stream-ordered
+// pool per call, given back to the driver at each synchronisation, cost up to milliseconds).
+static cudaError_t mass_sums(HydSim* h, double (&r)[5]) {
+    const int nb = 148;
+    if (!h->run_part) {
+        const cudaError_t e = cudaMalloc(&h->run_part, ((size_t)nb * 5 + 5) * sizeof(double));
+        if (e != cudaSuccess) return e;
+    }
+    k_mass_partial<<<nb, 256, 0, h->stream>>>(h->g, h->run_part);
+    k_mass_final<<<1, 160, 0, h->stream>>>(h->run_part, nb, h->run_part + nb * 5);
+    hyd_kernel_launches_add(2);
+    const cudaError_t e = cudaMemcpyAsync(r, h->run_part + nb * 5, sizeof r, cudaMemcpyDeviceToHost, h->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+}
+
 // Non-finite values in z, u, v, FS (the mass-balance kernels' count), on the handle's
 // stream; -1 on error.
 static long long count_nonfinite(HydSim* h) {
-    const int nb = 148;
-    if (!h->run_part && cudaMalloc(&h->run_part, ((size_t)nb * 5 + 5) * sizeof(double)) != cudaSuccess) return -1;
-    k_mass_partial<<<nb, 256, 0, h->stream>>>(h->g, h->run_part);
-    k_mass_final<<<1, 32, 0, h->stream>>>(h->run_part, nb, h->run_part + nb * 5);
-    hyd_kernel_launches_add(2);
     double r[5];
-    if (cudaMemcpyAsync(r, h->run_part + nb * 5, sizeof r, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
-        cudaStreamSynchronize(h->stream) != cudaSuccess)
-        return -1;
-    return (long long)r[4];
+    return mass_sums(h, r) == cudaSuccess ? (long long)r[4] : -1;
 }
 
 // An output time of hyd_run: t integral and a whole multiple of interval (Engine.py:398).
@@ -1410,22 +1423,39 @@ int hyd_checkpoint(hyd_handle h, int restore) {
     return set_clock(h, h->t);  // synchronises the stream
 }
 
-// The steady residual; with `status`, the device status word is read back in the same
-// synchronisation (the quasi-steady period's warm steps run without a check of their own).
-static int steady_residual(HydSim* h, int snapshot, double* out, unsigned* status) {
+// The steady residual's launch on the handle's stream, its results left at *tot (with
+// `snapshot`, the current u, v, z become the snapshot).
+static int residual_launch(HydSim* h, int snapshot, double** tot_out) {
     const size_t field = (size_t)(h->N + 3) * h->pitch;
     const int nb = 2 * 148;
     if (!h->res_buf) {
-        CUDA_TRY(cudaMalloc(&h->res_buf, (3 * field + (size_t)nb * 4 + 4) * sizeof(double)));
+        // three snapshot fields, the CTAs' sums, five results and the finished-CTA count
+        const size_t n = 3 * field + (size_t)nb * 4 + 6;
+        double* p = nullptr;
+        CUDA_TRY(cudaMalloc(&p, n * sizeof(double)));
+        const cudaError_t e = cudaMemsetAsync(p + n - 1, 0, sizeof(double), h->stream);
+        if (e != cudaSuccess) cudaFree(p);
+        CUDA_TRY(e);
+        h->res_buf = p;
         h->res_valid = 0;
     }
     double *u0 = h->res_buf, *v0 = u0 + field, *z0 = v0 + field, *part = z0 + field, *tot = part + (size_t)nb * 4;
-    launch_steady_residual(h->g, u0, v0, z0, snapshot, part, nb, tot, h->stream);
+    launch_steady_residual(h->g, u0, v0, z0, snapshot, part, nb, reinterpret_cast<unsigned*>(tot + 5), tot, h->stream);
     CUDA_TRY(cudaGetLastError());
-    double sums[4];
+    *tot_out = tot;
+    return HYD_OK;
+}
+
+// The steady residual; with `status`, the device status word is read back in the same
+// synchronisation (the quasi-steady period's warm steps run without a check of their own).
+static int steady_residual(HydSim* h, int snapshot, double* out, unsigned* status) {
+    double* tot = nullptr;
+    const int rc = residual_launch(h, snapshot, &tot);
+    if (rc) return rc;
+    double sums[5];
     CUDA_TRY(cudaMemcpyAsync(sums, tot, sizeof sums, cudaMemcpyDeviceToHost, h->stream));
-    if (status) CUDA_TRY(cudaMemcpyAsync(status, h->g.status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (status) *status = (unsigned)sums[4];
     if (!h->res_valid || !(sums[1] > 0) || !(sums[3] > 0)) {
         out[0] = out[1] = HUGE_VAL;  // no snapshot yet, no wet cell or no flow: not steady
     } else {
@@ -1468,17 +1498,27 @@ int hyd_quasi_steady_period(hyd_handle h, double period, int warm, int min_warm,
         ok = 0;
         int e = hyd_set_time(h, t_end - warm * dT);
         if (e) return e;
-        double r[2], t;
-        e = hyd_steady_residual(h, 1, r, 2);
-        if (e) return e;
-        for (int k = 1; k < warm; k++) {
-            e = hyd_step(h, 1, 0, &t);
-            if (e) return e;
+        double r[2], t, *tot;
+        // no residual is read before the min_warm-th step: until then nothing waits for the
+        // device, and the state before that step is the snapshot it is compared with
+        for (int k = 0; k < warm; k++) {
+            if (k > 0) {
+                e = hyd_step(h, 1, 0, &t);
+                if (e) return e;
+            }
+            if (k < min_warm) {
+                if (k == min_warm - 1) {
+                    e = residual_launch(h, 1, &tot);
+                    if (e) return e;
+                    h->res_valid = 1;
+                }
+                continue;
+            }
             unsigned st = 0;
             e = steady_residual(h, 1, r, &st);
             if (e) return e;
             if (st & HYD_ST_SEG_OVERFLOW) break;
-            if (k >= min_warm && r[0] < gate && r[1] < gate) {
+            if (r[0] < gate && r[1] < gate) {
                 double mb[5];
                 e = hyd_mass_balance(h, mb, 5);
                 if (e) return e;
@@ -1551,16 +1591,8 @@ int hyd_synchronize(hyd_handle h) {
 int hyd_mass_balance(hyd_handle h, double* out, int n) {
     if (!h || !out || n < 5) return fail(HYD_EINVAL, "need 5 output slots");
     CUDA_TRY(cudaSetDevice(h->device));
-    const int nb = 148;
-    double* part = nullptr;
-    CUDA_TRY(cudaMallocAsync(&part, (size_t)nb * 5 * 8 + 5 * 8, h->stream));
-    k_mass_partial<<<nb, 256, 0, h->stream>>>(h->g, part);
-    k_mass_final<<<1, 32, 0, h->stream>>>(part, nb, part + nb * 5);
-    hyd_kernel_launches_add(2);
     double r[5];
-    CUDA_TRY(cudaMemcpyAsync(r, part + nb * 5, sizeof r, cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaFreeAsync(part, h->stream));
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    CUDA_TRY(mass_sums(h, r));
     const double area = h->P.dX * h->P.dY;
     out[0] = r[0] * area;
     out[1] = r[1] * area;
@@ -1610,7 +1642,7 @@ int hyd_mass_balance_noalloc(hyd_handle h, int nblocks, double* out, int n) {
         if (e != cudaSuccess) return fail(HYD_ECUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
     }
     k_mass_partial<<<nblocks, 256, 0, h->stream>>>(h->g, part);
-    k_mass_final<<<1, 32, 0, h->stream>>>(part, nblocks, part + nblocks * 5);
+    k_mass_final<<<1, 160, 0, h->stream>>>(part, nblocks, part + nblocks * 5);
     hyd_kernel_launches_add(2);
     CUDA_TRY(cudaGetLastError());
     double r[5];

@@ -397,10 +397,11 @@ void launch_bed_reset(const DevGrid& g, cudaStream_t s);
 // the depths and face depths re-derived around them
 void launch_add_levels(const DevGrid& g, const DevParams& p, const float* du, const float* dv, const float* dz,
                        int i0, int j0, int rows, int cols, long long ld, cudaStream_t s);
-// hyd_steady_residual: per-CTA sums over the wet cells (4 per CTA), then the totals in
-// out[0..3] added in CTA order; snapshot: u0, v0, z0 = u, v, z afterwards
+// hyd_steady_residual: per-CTA sums over the wet cells (4 per CTA, into part), their totals in
+// out[0..3] added in a fixed order, the device status word in out[4]; *count is zero between
+// launches; snapshot: u0, v0, z0 = u, v, z afterwards
 void launch_steady_residual(const DevGrid& g, double* u0, double* v0, double* z0, int snapshot, double* part,
-                            int nblocks, double* out, cudaStream_t s);
+                            int nblocks, unsigned* count, double* out, cudaStream_t s);
 long long hyd_kernel_launches_add(long long n);
 
 // Batched launches (k_grid.cu, k_sweep.cu): one launch for every member of a batch, each

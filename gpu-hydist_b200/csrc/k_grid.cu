@@ -2207,51 +2207,70 @@ __global__ void k_add_levels_faces(DevGrid g, int i0, int j0, int rows, int cols
 }
 
 // hyd_steady_residual: sums over the wet cells of 2..N x 2..M of (u - u0)^2 + (v - v0)^2,
-// u^2 + v^2, (z - z0)^2 and H_moi^2, per CTA; with snapshot, the cell's u, v, z are copied
-// to u0, v0, z0 after they are read.
-__global__ void k_resid_partial(DevGrid g, double* __restrict__ u0, double* __restrict__ v0, double* __restrict__ z0,
-                                int snapshot, double* __restrict__ part) {
+// u^2 + v^2, (z - z0)^2 and H_moi^2 into out[0..3], and the device status word into out[4];
+// with snapshot, the cell's u, v, z are copied to u0, v0, z0 after they are read.  One warp
+// per row over the row's span of cells that can be wet (config 2: 4 % of the grid); each CTA's
+// sums go to part, and the last CTA to finish (counted at *count, which it resets) adds them,
+// thread by thread and then as a tree, so the order is fixed.  A cell at a time over the whole
+// grid, its row and column by 64-bit divisions, with one thread adding the CTAs' sums, took
+// about 150 us on config 2; this is bound by its launch and its dependent loads (under 10 us).
+__global__ void __launch_bounds__(256) k_resid(DevGrid g, double* __restrict__ u0, double* __restrict__ v0,
+                                               double* __restrict__ z0, int snapshot, double* part, unsigned* count,
+                                               double* out) {
     __shared__ double sh[4][256];
-    const int tid = threadIdx.x;
+    __shared__ int s_last;
+    const int tid = threadIdx.x, lane = tid & 31;
     double a = 0, b = 0, c = 0, d = 0;
-    const int W = g.M - 1;
-    const long long ncell = (long long)(g.N - 1) * W;
-    for (long long q = (long long)blockIdx.x * blockDim.x + tid; q < ncell; q += (long long)gridDim.x * blockDim.x) {
-        const int i = 2 + (int)(q / W), j = 2 + (int)(q % W);
-        const int gp = i * g.P + j;
-        if (g.khouot[gp] != 0) continue;
-        const double u = g.u[gp], v = g.v[gp], z = g.z[gp], H = g.H_moi[gp];
-        const double du = u - u0[gp], dv = v - v0[gp], dz = z - z0[gp];
-        a += du * du + dv * dv;
-        b += u * u + v * v;
-        c += dz * dz;
-        d += H * H;
-        if (snapshot) {
-            u0[gp] = u;
-            v0[gp] = v;
-            z0[gp] = z;
+    for (int i = 2 + ((blockIdx.x * blockDim.x + tid) >> 5); i <= g.N; i += (gridDim.x * blockDim.x) >> 5) {
+        const int lo = max(g.rlo[i], 2), hi = min(g.rhi[i], g.M);
+        for (int j = lo + lane; j <= hi; j += 32) {
+            const int gp = i * g.P + j;
+            const double u = g.u[gp], v = g.v[gp], z = g.z[gp], H = g.H_moi[gp];
+            const double du = u - u0[gp], dv = v - v0[gp], dz = z - z0[gp];
+            if (g.khouot[gp] != 0) continue;
+            a += du * du + dv * dv;
+            b += u * u + v * v;
+            c += dz * dz;
+            d += H * H;
+            if (snapshot) {
+                u0[gp] = u;
+                v0[gp] = v;
+                z0[gp] = z;
+            }
         }
     }
-    sh[0][tid] = a;
-    sh[1][tid] = b;
-    sh[2][tid] = c;
-    sh[3][tid] = d;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (tid < w)
-            for (int k = 0; k < 4; k++) sh[k][tid] += sh[k][tid + w];
+    auto tree = [&]() {
+        sh[0][tid] = a;
+        sh[1][tid] = b;
+        sh[2][tid] = c;
+        sh[3][tid] = d;
         __syncthreads();
-    }
-    if (tid == 0)
+        for (int w = 128; w > 0; w >>= 1) {
+            if (tid < w)
+                for (int k = 0; k < 4; k++) sh[k][tid] += sh[k][tid + w];
+            __syncthreads();
+        }
+    };
+    tree();
+    if (tid == 0) {
         for (int k = 0; k < 4; k++) part[blockIdx.x * 4 + k] = sh[k][0];
-}
-
-__global__ void k_resid_final(const double* __restrict__ part, int nblocks, double* __restrict__ out) {
-    if (threadIdx.x != 0) return;
-    double acc[4] = {0, 0, 0, 0};
-    for (int b = 0; b < nblocks; b++)
-        for (int k = 0; k < 4; k++) acc[k] += part[b * 4 + k];
-    for (int k = 0; k < 4; k++) out[k] = acc[k];
+        __threadfence();
+        s_last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    a = b = c = d = 0;
+    for (int q = tid; q < (int)gridDim.x; q += 256) {
+        a += __ldcg(part + 4 * q);
+        b += __ldcg(part + 4 * q + 1);
+        c += __ldcg(part + 4 * q + 2);
+        d += __ldcg(part + 4 * q + 3);
+    }
+    tree();
+    if (tid < 4) out[tid] = sh[tid][0];
+    if (tid == 4) out[4] = (double)*g.status;
+    if (tid == 0) *count = 0u;
 }
 
 // Feedback set-up: h0 = h - dH (so that h = h0 + dH holds now), no compensation yet.
@@ -2587,10 +2606,9 @@ void launch_add_levels(const DevGrid& g, const DevParams& p, const float* du, co
 }
 
 void launch_steady_residual(const DevGrid& g, double* u0, double* v0, double* z0, int snapshot, double* part,
-                            int nblocks, double* out, cudaStream_t s) {
-    k_resid_partial<<<nblocks, 256, 0, s>>>(g, u0, v0, z0, snapshot, part);
-    k_resid_final<<<1, 32, 0, s>>>(part, nblocks, out);
-    hyd_kernel_launches_add(2);
+                            int nblocks, unsigned* count, double* out, cudaStream_t s) {
+    k_resid<<<nblocks, 256, 0, s>>>(g, u0, v0, z0, snapshot, part, count, out);
+    hyd_kernel_launches_add(1);
 }
 
 // Up to kPutDoubles values carried in the launch's parameters into dst[0..n): a small

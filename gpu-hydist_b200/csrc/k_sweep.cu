@@ -16,45 +16,39 @@
 //      (replaces the reference's serial Thomas sweep, UVZSolver_multithread.cu:203-228)
 //   D  the solution scattered to t_z / t_u (t_v) with the reference's boundary formulas.
 //
-// One persistent kernel per sweep: a 512-thread CTA per SM takes every G-th line, one
-// per warp.  A short line (at most 3 rows per lane) is swept by its warp alone; a long
-// line by the whole CTA in shared memory sized for the longest line the grid can hold (a
-// global scratch region per CTA beyond that).  A short line's solve is its warp's: lanes
-// eliminate chunks of rows, the chunk ends are solved by shuffle-only cyclic reduction; a
-// long line's adds a level (up to 256 threads eliminate chunks, one warp solves the
-// chunk-end system as above).
+// One persistent kernel per sweep: a 512-thread CTA per SM takes every G-th line, 16 at a time,
+// one warp setting up each.  The lines are then swept side by side by teams of warps, a
+// team's share of the 16 warps by its line's rows, as many lines at once as their rows fit
+// the shared memory (a global scratch region per CTA for a line that does not fit at all).
+// How a line is solved depends on its rows alone, not on its team: up to about 480 rows 32
+// chunks eliminated by one warp whose chunk ends are solved by shuffle-only cyclic reduction,
+// beyond that a level more (up to 256 chunks, then one warp on the chunk-end system as
+// above); so a line's values are the same bits in every launch shape.
 // In the column sweeps the cell-local coefficients come precomputed, stored column-major
 // so that a column reads them contiguously (k_coef_bnd<0>, k_coef_fsj).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "hydist_dev.cuh"
 
 namespace {
 
 constexpr int kTL = 512;         // threads of a sweep CTA
-constexpr int kWL = kTL / 32;    // lines per group (one per warp)
-// A warp's shared-memory slice holds kRowW rows (9 per lane).  Which lines a warp sweeps
-// alone is chosen per launch: with at most one group of lines per CTA, lines of at most
-// kRowShort rows (kRowShortF for sediment), the rest by the whole CTA (a long line then
-// costs the CTA less time than a warp would take); with more lines than that, every line
-// that fits the slice, so that a CTA's many medium lines run side by side.
+constexpr int kWL = kTL / 32;    // lines per group (one warp sets up each)
+// Shared memory asked for beyond the longest line: `wide`, room for every line of a group with
+// up to kRowW rows side by side; else up to kRowSlice rows (more of the SM's on-chip memory
+// left to L1).
 constexpr int kRowW = 288;
-constexpr int kRowShort = 96;
-constexpr int kRowShortF = 64;
+constexpr int kRowSlice = 96;
 // continuity coefficients (a, c, d) of the first and last cell of every segment of a
-// hydrodynamic line, kept for the extraction: 6 doubles per segment
+// hydrodynamic line, kept for the extraction: 6 values per segment
 constexpr int kEnds = 6 * HYD_SEGL;
-constexpr int kWarpHydro = 4 * kRowW + kEnds;  // doubles per warp (the largest slice)
-constexpr int kWarpFs = 4 * kRowW;
-constexpr int kRowSlice = 96;  // rows of a slice when warps take lines of up to kRowShort (kRowShortF) rows
-// rows of a warp's slice for a launch whose warps take lines of up to roww rows
-__host__ __device__ inline int slice_rows(int roww) { return roww > kRowSlice ? kRowW : kRowSlice; }
-static_assert(kRowW % 32 == 0 && (kRowW / 32) % 2 == 1, "a warp solve pads R <= kRowW rows to 32 chunk_len(R, 32) <= kRowW");
 
-// A group of threads that sweeps one line: a warp, or a whole CTA for a long line.
-// WarpG::exchange() gives lane t the values v of lanes t - h (lo) and t + h (hi).
+// A warp's threads setting up a line.  exchange() gives lane t the values v of lanes t - h (lo)
+// and t + h (hi).
 struct WarpG {
     static constexpr int size = 32;
     __device__ static __forceinline__ int rank() { return threadIdx.x & 31; }
@@ -69,16 +63,30 @@ struct WarpG {
     }
 };
 
-struct BlockG {
-    static constexpr int size = kTL;
-    __device__ static __forceinline__ int rank() { return threadIdx.x; }
-    __device__ static __forceinline__ void sync() { __syncthreads(); }
+// The threads that sweep one line: a warp by itself, or a team.
+struct WarpTeam {
+    static constexpr int size = 32;
+    const int rank = threadIdx.x & 31;
+    __device__ __forceinline__ void sync() const { __syncwarp(); }
+};
+
+// The warps [first, first + size / 32) of the CTA sweeping one line.  Teams of several warps
+// meet at a hardware barrier of their own (1 + first / 2: two teams of two warps or more start
+// at least two warps apart; barrier 0 is the CTA's).
+struct Team {
+    int size, rank, bar;
+    __device__ __forceinline__ Team(int first, int warps)
+        : size(32 * warps), rank((int)threadIdx.x - 32 * first), bar(1 + first / 2) {}
+    __device__ __forceinline__ void sync() const {
+        if (size == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(size) : "memory");
+    }
 };
 
 // Chunk length for R rows over T threads: at least 3 and odd (odd strides keep the
 // chunk-strided shared-memory accesses free of bank conflicts).
 __host__ __device__ inline int chunk_len(int R, int T) {
-    int m = (R + T - 1) / T;
+    int m = (int)((unsigned)(R + T - 1) / (unsigned)T);
     if (m < 3) m = 3;
     if ((m & 1) == 0) m++;
     return m;
@@ -207,19 +215,23 @@ __device__ __forceinline__ void solve_warp(R* A, R* B, R* C, R* D, int m) {
     __syncwarp();
 }
 
-// How a group of threads solves R rows: t1 threads with chunks of m rows.  t1 == 32: one
-// warp (solve_warp).  t1 > 32: two levels (solve_block): the 2 t1 chunk-end rows form a
-// tridiagonal system that one warp solves in chunks of m2 = chunk_len(2 t1, 32) rows.
-// The plan minimises the serial depth, about 3 m + 6 for one warp and 3 m + 3 m2 + 10
-// for two levels (their two CTA barriers counted as two steps each).
+// How R rows are solved: t1 chunks of m rows.  t1 == 32: one warp (solve_warp).  t1 > 32: two
+// levels (solve_two): the 2 t1 chunk-end rows form a tridiagonal system that one warp solves
+// in chunks of m2 = chunk_len(2 t1, 32) rows.  The plan minimises the serial depth, about
+// 3 m + 6 for one warp and 3 m + 3 m2 + 10 for two levels (their two barriers counted as two
+// steps each).
 struct SolvePlan {
     int t1, m;
+    __host__ __device__ int rows() const { return t1 * m; }                                   // padded
+    __host__ __device__ int red() const { return t1 > 32 ? 32 * chunk_len(2 * t1, 32) : 0; }  // reduced rows
 };
 constexpr int kRedRows = 32 * 17;  // reduced rows of the largest two-level plan (t1 = 256)
 __host__ __device__ inline SolvePlan solve_plan(int R, int max_t1) {
     SolvePlan best{32, chunk_len(R, 32)};
     int depth = 3 * best.m + 6;
-    for (int t1 = 64; t1 <= max_t1 && t1 <= 256; t1 <<= 1) {
+#pragma unroll
+    for (int t1 = 64; t1 <= 256; t1 <<= 1) {  // unrolled: the divisions become shifts
+        if (t1 > max_t1) break;
         const int m1 = chunk_len(R, t1), m2 = chunk_len(2 * t1, 32);
         const int d = 3 * m1 + 3 * m2 + 10;
         if (d < depth) {
@@ -230,14 +242,13 @@ __host__ __device__ inline SolvePlan solve_plan(int R, int max_t1) {
     return best;
 }
 
-// Two-level solve by a CTA (rows [0, t1 m)); red holds 4 kRedRows doubles.  Every thread
-// of the CTA calls it.  On return B[r] holds x[r].
-template <class R>
-__device__ __forceinline__ void solve_block(R* A, R* B, R* C, R* D, SolvePlan pl, R* red) {
-    const int t = threadIdx.x;
-    const int m2 = chunk_len(2 * pl.t1, 32);
-    R *rA = red, *rB = red + kRedRows, *rC = red + 2 * kRedRows, *rD = red + 3 * kRedRows;
-    if (t < pl.t1) {
+// Two-level solve by a team (rows [0, t1 m)); red holds 4 red() values.  Every thread of the
+// team calls it.  On return B[r] holds x[r].
+template <class R, class TM>
+__device__ __forceinline__ void solve_two(R* A, R* B, R* C, R* D, SolvePlan pl, R* red, const TM& tm) {
+    const int nr = pl.red();
+    R *rA = red, *rB = red + nr, *rC = red + 2 * nr, *rD = red + 3 * nr;
+    for (int t = tm.rank; t < pl.t1; t += tm.size) {
         const int s = t * pl.m, e = s + pl.m - 1;
         R v[6];
         chunk_reduce(A, B, C, D, s, e, v);
@@ -250,28 +261,28 @@ __device__ __forceinline__ void solve_block(R* A, R* B, R* C, R* D, SolvePlan pl
         rC[2 * t + 1] = v[4];
         rD[2 * t + 1] = v[5];
     }
-    for (int r = 2 * pl.t1 + t; r < 32 * m2; r += blockDim.x) {  // identity rows
+    for (int r = 2 * pl.t1 + tm.rank; r < nr; r += tm.size) {  // identity rows
         rA[r] = R(0);
         rB[r] = R(1);
         rC[r] = R(0);
         rD[r] = R(0);
     }
-    __syncthreads();
-    if (t < 32) solve_warp(rA, rB, rC, rD, m2);
-    __syncthreads();
-    if (t < pl.t1) {
+    tm.sync();
+    if (tm.rank < 32) solve_warp(rA, rB, rC, rD, nr / 32);
+    tm.sync();
+    for (int t = tm.rank; t < pl.t1; t += tm.size) {
         const int s = t * pl.m, e = s + pl.m - 1;
         chunk_back(A, B, C, D, s, e, rB[2 * t], rB[2 * t + 1]);
     }
-    __syncthreads();
+    tm.sync();
 }
 
-// Serial Thomas over the packed rows by the group's first thread, in the reference's
+// Serial Thomas over the packed rows by the team's first thread, in the reference's
 // operation order (tridiag, UVZSolver_multithread.cu:203-228); decoupled segments solve
 // exactly as separate systems.  Used to check the partitioned solver.
-template <class G, class R>
-__device__ __forceinline__ void solve_thomas(R* A, R* B, R* C, R* D, int rows) {
-    if (G::rank() == 0 && rows > 0) {
+template <class R, class TM>
+__device__ __forceinline__ void solve_thomas(R* A, R* B, R* C, R* D, int rows, const TM& tm) {
+    if (tm.rank == 0 && rows > 0) {
         R Ap = -C[0] / B[0], Bp = D[0] / B[0];
         C[0] = Ap;
         D[0] = Bp;
@@ -289,25 +300,22 @@ __device__ __forceinline__ void solve_thomas(R* A, R* B, R* C, R* D, int rows) {
             B[i] = x;
         }
     }
-    G::sync();
+    tm.sync();
 }
 
-// Solve of a line's packed system (rows padded with identity rows to pl.t1 * pl.m) by
-// group G: one warp (a warp group, or a CTA's first warp with the others waiting), or
-// the two-level solve of a CTA.
-template <class G, int SOLVER, class R>
-__device__ __forceinline__ void solve_line(R* A, R* B, R* C, R* D, SolvePlan pl, int rows, R* red) {
+// Solve of a line's packed system (rows padded with identity rows to pl.rows()) by a team.
+template <int SOLVER, class R, class TM>
+__device__ __forceinline__ void solve_line(R* A, R* B, R* C, R* D, SolvePlan pl, int rows, R* red, const TM& tm) {
+    constexpr bool one = std::is_same<TM, WarpTeam>::value;  // its lines are never long enough for two levels
     if (SOLVER == 0) {
-        if (G::size == 32) {
-            solve_warp(A, B, C, D, pl.m);
-        } else if (pl.t1 == 32) {
-            if (threadIdx.x < 32) solve_warp(A, B, C, D, pl.m);
-            G::sync();
+        if (one || pl.t1 == 32) {
+            if (tm.rank < 32) solve_warp(A, B, C, D, pl.m);
+            if (tm.size > 32) tm.sync();
         } else {
-            solve_block(A, B, C, D, pl, red);
+            solve_two(A, B, C, D, pl, red, tm);
         }
     } else {
-        solve_thomas<G, R>(A, B, C, D, rows);
+        solve_thomas(A, B, C, D, rows, tm);
     }
 }
 
@@ -412,18 +420,18 @@ __device__ __forceinline__ void hydro_setup(const DevGrid& g, const DevParams& p
     G::sync();
 }
 
-// Phases A-D of one line by group G.  Rows A, B, Cc, D hold at least pl.t1 * pl.m
-// entries, ends kEnds; red: the two-level solve's reduced rows.
+// Phases A-D of one line by a team.  Rows A, B, Cc, D hold at least pl.rows() entries, ends
+// kEnds; red: the two-level solve's reduced rows.
 // R = float: the mixed form.  Its coefficients (k_coef_bnd's FP32 arrays) are those of the
 // level increment dz = z' - z: the continuity right-hand side d2 - z and the momentum
 // f5 - f4 (z_k - z_k+1), so that the same rows solve for (dz, u) in FP32; the prescribed
 // levels enter as increments, and the new level is z + dz in FP64.
-template <int DIR, int SOLVER, class G, class R>
+template <int DIR, int SOLVER, class R, class TM>
 __device__ __forceinline__ void hydro_body(const DevGrid& g, const DevParams& p, int line, const LineShared& sg,
-                                           R* A, R* B, R* Cc, R* D, R* ends, R* red, SolvePlan pl) {
+                                           R* A, R* B, R* Cc, R* D, R* ends, R* red, SolvePlan pl, const TM& tm) {
     constexpr bool MIX = sizeof(R) == sizeof(float);
-    constexpr int T = G::size;
-    const int tid = G::rank();
+    const int T = tm.size;
+    const int tid = tm.rank;
     const int N = g.N, M = g.M, P = g.P;
     const int L = DIR == 0 ? N : M;
     (void)M;
@@ -452,7 +460,7 @@ __device__ __forceinline__ void hydro_body(const DevGrid& g, const DevParams& p,
             d = rowCr<R>(g, 2)[pos];
         }
     };
-    for (int r = Rn + tid; r < pl.t1 * pl.m; r += T) {  // identity rows up to the solver's rows
+    for (int r = Rn + tid; r < pl.rows(); r += T) {  // identity rows up to the solver's rows
         A[r] = R(0);
         B[r] = R(1);
         Cc[r] = R(0);
@@ -542,7 +550,7 @@ __device__ __forceinline__ void hydro_body(const DevGrid& g, const DevParams& p,
             D[r0 + rel + 1] = dn;
         }
     }
-    G::sync();
+    tm.sync();
 
     // ---- B2: segment end rows (_calculate_matrix_coeff 469-592) and decoupling
     if (tid < nseg && sg.sn[tid] >= 0) {
@@ -567,10 +575,10 @@ __device__ __forceinline__ void hydro_body(const DevGrid& g, const DevParams& p,
         A[rowF] = R(0);
         Cc[rowL] = R(0);
     }
-    G::sync();
+    tm.sync();
 
     // ---- C: solve
-    solve_line<G, SOLVER, R>(A, B, Cc, D, pl, Rn, red);
+    solve_line<SOLVER, R>(A, B, Cc, D, pl, Rn, red, tm);
 
     // ---- D: extract (_uzSolver_extract_solution 668-723 / _vzSolver_extract_solution 595-665)
     const R* x = B;
@@ -636,80 +644,142 @@ struct OneGridLines {
     __device__ __forceinline__ const DevParams& params(int) const { return p; }
 };
 
+// Which of a group's lines are swept now, and by whom: computed by every warp alike.  Lane l
+// of a warp holds the values of shared memory line l's sweep needs.  Of the lines still to do
+// (todo), those whose needs added up in order fit `cap` are taken; line l gets warps [start,
+// end) of the 16, at least one, the others in proportion to the needs.  (Few instructions and
+// few dependent shuffles: this is on every CTA's path, once per 16 lines.)
+struct TeamPick {
+    unsigned sel;      // lines of this round (0: the first line left does not fit at all)
+    int line;          // this warp's line
+    int first, warps;  // its team
+    int off;           // where the line's region of the shared memory starts
+};
+__device__ __forceinline__ TeamPick pick_team(unsigned todo, int need, int cap) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool in = (todo >> lane) & 1u;  // todo has no bit beyond the group's kWL lines
+    int sum = in ? need : 0;
+#pragma unroll
+    for (int o = 1; o < kWL; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    TeamPick t;
+    t.sel = __ballot_sync(0xffffffffu, in && sum <= cap);
+    t.line = t.first = t.warps = t.off = 0;
+    if (t.sel == 0) return t;
+    const int last = 31 - __clz(t.sel);
+    const int total = __shfl_sync(0xffffffffu, sum, last);
+    // the spare warps up to this line by the needs up to it; all of them up to the last line
+    // (the product is monotone in sum and at most spare, whatever the reciprocal's rounding)
+    const int spare = kWL - __popc(t.sel);
+    const int share = lane >= last ? spare : min((int)((float)(spare * sum) * __frcp_rn((float)total)), spare);
+    int prev = __shfl_up_sync(0xffffffffu, share, 1);
+    if (lane == 0) prev = 0;
+    const int before = __popc(t.sel & ((1u << lane) - 1u));
+    const int start = before + prev, end = before + 1 + share;
+    t.line = 31 - __clz(__ballot_sync(0xffffffffu, ((t.sel >> lane) & 1u) && start <= w));
+    const int v = __shfl_sync(0xffffffffu, (sum - need) << 10 | end << 5 | start, t.line);
+    t.first = v & 31;
+    t.warps = ((v >> 5) & 31) - t.first;
+    t.off = v >> 10;
+    return t;
+}
+
 // Fused sweep of one direction.  CTA b takes lines b, b + G, b + 2G, ... (G = gridDim.x)
-// in groups of 16, one line per warp.  Every warp sets its line up; a warp whose line is
-// short (at most roww rows) sweeps it alone in its own slice of shared memory; then the
-// whole CTA sweeps the group's long lines one after another in the full shared memory
-// (RB rows; a CTA's region of global scratch beyond that).
-// Adjacent long lines (a wet band) fall on different CTAs.  Warps with nothing to sweep
-// wait at the CTA barriers rather than exit: the warp-synchronous steps of a warp whose
-// sibling warps had exited were measured an order of magnitude slower on B200.
+// in groups of 16; every warp sets a line up, then the group's lines are swept by teams
+// (pick_team), in as many rounds as their rows need of the shared memory; when no line has more
+// than kRowSlice rows, each by its own warp in a slice of its own (short lines gain nothing
+// from more warps, and the picking and the barriers cost them 1 us of 9).  A line of more than
+// RB rows, or that does not fit alone, is swept by the whole CTA in its region of global
+// scratch.  Adjacent long lines (a wet band) fall on different CTAs.
+// Against one warp per short line and then the whole CTA on one long line after another
+// (the lines of more than 96 rows of a grid with at most 16 lines per CTA): the 2047 rows of
+// about 240 solver rows of a 2048 x 2048 reach 88 -> 29 us (the solve of a line up to 480 rows
+// is one warp's, so the other 15 waited), the 99-row lines of a 400 x 60 channel 20 -> 12; one
+// long column among short ones, as on a 1048 x 980 reach, 15.1 -> 14.9.
+// Warps with nothing to sweep wait at the CTA barriers rather than exit: the
+// warp-synchronous steps of a warp whose sibling warps had exited were measured an order of
+// magnitude slower on B200.
 template <int DIR, int SOLVER, class R, class Lines>
-__device__ __forceinline__ void hydro_sweep_loop(const Lines& lines, int RB, double* gscr_d, int RG, int roww) {
+__device__ __forceinline__ void hydro_sweep_loop(const Lines& lines, int cap, int RB, double* gscr_d, int RG) {
     constexpr bool MIX = sizeof(R) == sizeof(float);
     extern __shared__ double dyn_smem_d[];
     R* dyn_smem = reinterpret_cast<R*>(dyn_smem_d);
-    R* gscr = reinterpret_cast<R*>(gscr_d);
     __shared__ LineShared sgw[kWL];
-    __shared__ int s_long[kWL], s_mem[kWL], s_line[kWL];
-    __shared__ int s_nlong;
-    __shared__ R s_red[4 * kRedRows];  // reduced rows of the two-level solve
-    const int w = threadIdx.x >> 5;
+    __shared__ int s_mem[kWL], s_line[kWL];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nlines = lines.count();
     const int G = gridDim.x;
     for (int j0 = 0; (int)blockIdx.x + j0 * G < nlines; j0 += kWL) {
         const int li = blockIdx.x + (j0 + w) * G;
         LineShared& sg = sgw[w];
-        int m = 0, line = 0;
-        if (li < nlines) lines.at(li, m, line);
-        if (threadIdx.x == 0) s_nlong = 0;
-        if ((threadIdx.x & 31) == 0) {
-            s_mem[w] = m;
-            s_line[w] = line;
-        }
-        if (li < nlines) hydro_setup<DIR, WarpG, MIX>(lines.grid(m), lines.params(m), line, sg);  // warp-uniform
-        __syncthreads();
-        if (li < nlines && sg.nseg > 0) {
-            if (sg.R > roww) {
-                if ((threadIdx.x & 31) == 0) s_long[atomicAdd(&s_nlong, 1)] = w;
-            } else {
-                const int wr = slice_rows(roww);
-                R* A = dyn_smem + w * (4 * wr + kEnds);
-                R* B = A + wr;
-                R* Cc = B + wr;
-                R* D = Cc + wr;
-                hydro_body<DIR, SOLVER, WarpG, R>(lines.grid(m), lines.params(m), line, sg, A, B, Cc, D, D + wr,
-                                                  nullptr, SolvePlan{32, chunk_len(sg.R, 32)});
+        if (li < nlines) {  // warp-uniform
+            int m = 0, line = 0;
+            lines.at(li, m, line);
+            if (lane == 0) {
+                s_mem[w] = m;
+                s_line[w] = line;
             }
+            hydro_setup<DIR, WarpG, MIX>(lines.grid(m), lines.params(m), line, sg);
+        } else if (lane == 0) {
+            sg.nseg = sg.R = 0;
         }
         __syncthreads();
-        const int nl = s_nlong;
-        for (int q = 0; q < nl; q++) {
-            const int wl = s_long[q];
-            const LineShared& sl = sgw[wl];
-            const int lm = s_mem[wl];
-            const SolvePlan pl = solve_plan(sl.R, SOLVER == 0 ? 256 : 32);
-            const bool fits = pl.t1 * pl.m <= RB;
-            const int rs = fits ? RB : RG;
-            R* A = fits ? dyn_smem : gscr + (size_t)blockIdx.x * (4 * (size_t)RG + kEnds);
-            R* B = A + rs;
-            R* Cc = B + rs;
-            R* D = Cc + rs;
-            hydro_body<DIR, SOLVER, BlockG, R>(lines.grid(lm), lines.params(lm), s_line[wl], sl, A, B, Cc, D, D + rs,
-                                               s_red, pl);
-            __syncthreads();  // the slices and sgw are reused
+        const LineShared& mine = sgw[lane & (kWL - 1)];
+        if (!__any_sync(0xffffffffu, mine.R > kRowSlice)) {  // the same in every warp
+            if (sg.nseg > 0) {
+                R* A = dyn_smem + w * (4 * kRowSlice + kEnds);
+                hydro_body<DIR, SOLVER, R>(lines.grid(s_mem[w]), lines.params(s_mem[w]), s_line[w], sg, A, A + kRowSlice,
+                                           A + 2 * kRowSlice, A + 3 * kRowSlice, A + 4 * kRowSlice, (R*)nullptr,
+                                           SolvePlan{32, chunk_len(sg.R, 32)}, WarpTeam());
+            }
+            __syncthreads();
+            continue;
+        }
+        const SolvePlan mp = solve_plan(mine.R, SOLVER == 0 ? 256 : 32);
+        const int need = 4 * mp.rows() + kEnds + 4 * mp.red() + (mp.rows() > RB ? cap : 0);
+        unsigned todo = __ballot_sync(0xffffffffu, lane < kWL && mine.nseg > 0);
+        while (todo) {
+            TeamPick t = pick_team(todo, need, cap);
+            const bool global = t.sel == 0;  // the first line left, by the whole CTA
+            if (global) {
+                t.line = __ffs(todo) - 1;
+                t.sel = 1u << t.line;
+                t.warps = kWL;
+            }
+            const LineShared& sl = sgw[t.line];
+            const Team tm(t.first, t.warps);
+            const int pv = __shfl_sync(0xffffffffu, mp.m << 10 | mp.t1, t.line);
+            const SolvePlan pl{pv & 1023, pv >> 10};
+            const int lm = s_mem[t.line], ln = s_line[t.line];
+            // two calls, so that the first one's rows are known to be shared memory (through
+            // generic addresses the long columns' sweep took 15.6 instead of 14.8 us)
+            if (__builtin_expect(!global, 1)) {
+                const int P = pl.rows();
+                R* A = dyn_smem + t.off;
+                R* ends = A + 4 * P;
+                hydro_body<DIR, SOLVER, R>(lines.grid(lm), lines.params(lm), ln, sl, A, A + P, A + 2 * P, A + 3 * P, ends,
+                                           ends + kEnds, pl, tm);
+            } else {
+                R* A = reinterpret_cast<R*>(gscr_d) + (size_t)blockIdx.x * (4 * (size_t)RG + kEnds);
+                hydro_body<DIR, SOLVER, R>(lines.grid(lm), lines.params(lm), ln, sl, A, A + RG, A + 2 * RG, A + 3 * RG,
+                                           A + 4 * RG, dyn_smem, pl, tm);
+            }
+            todo &= ~t.sel;
+            __syncthreads();  // the regions and sgw are reused
         }
     }
 }
 
 template <int DIR, int SOLVER, class R>
-__global__ void __launch_bounds__(kTL, 1) k_hydro_sweep(DevGrid g, DevParams p, int startidx, int endidx, int RB,
-                                                     double* gscr_d, int RG, int roww) {
-    hydro_sweep_loop<DIR, SOLVER, R>(OneGridLines{g, p, startidx, endidx - startidx + 1}, RB, gscr_d, RG, roww);
+__global__ void __launch_bounds__(kTL, 1) k_hydro_sweep(DevGrid g, DevParams p, int startidx, int endidx, int cap, int RB,
+                                                     double* gscr_d, int RG) {
+    hydro_sweep_loop<DIR, SOLVER, R>(OneGridLines{g, p, startidx, endidx - startidx + 1}, cap, RB, gscr_d, RG);
 }
 template <int DIR, int SOLVER, class R>
-__global__ void __launch_bounds__(kTL, 1) k_hydro_sweep_b(BatchLines bl, int RB, double* gscr_d, int RG, int roww) {
-    hydro_sweep_loop<DIR, SOLVER, R>(bl, RB, gscr_d, RG, roww);
+__global__ void __launch_bounds__(kTL, 1) k_hydro_sweep_b(BatchLines bl, int cap, int RB, double* gscr_d, int RG) {
+    hydro_sweep_loop<DIR, SOLVER, R>(bl, cap, RB, gscr_d, RG);
 }
 
 // ---- sediment sweeps --------------------------------------------------------------
@@ -884,17 +954,18 @@ __device__ __forceinline__ void fs_setup(const DevGrid& g, const DevParams& p, i
 // and _FSi/_FSj_extract_solution, Sediment_Transport.cu:62-340, driven by Scan_FSi/
 // Scan_FSj and FSi/FSj_extract_solution 570-618).  DIR 0: FSj (line = column j, cells
 // i), DIR 1: FSi (line = row i, cells j).
-template <int DIR, int SOLVER, class G, class R>
+template <int DIR, int SOLVER, class R, class TM>
 __device__ __forceinline__ void fs_body(const DevGrid& g, const DevParams& p, int half, int line,
-                                        const LineShared& sg, R* A, R* B, R* Cc, R* D, R* red, SolvePlan pl) {
-    constexpr int T = G::size;
-    const int tid = G::rank();
+                                        const LineShared& sg, R* A, R* B, R* Cc, R* D, R* red, SolvePlan pl,
+                                        const TM& tm) {
+    const int T = tm.size;
+    const int tid = tm.rank;
     const int P = g.P;
     const int along = DIR == 0 ? P : 1;
     const int base = DIR == 0 ? line : line * P;
     (void)half;  // both rows are precomputed (k_coef_fsj, the state update's FSi terms)
     const int Rn = sg.R;
-    for (int r = Rn + tid; r < pl.t1 * pl.m; r += T) {  // identity rows up to the solver's rows
+    for (int r = Rn + tid; r < pl.rows(); r += T) {  // identity rows up to the solver's rows
         A[r] = R(0);
         B[r] = R(1);
         Cc[r] = R(0);
@@ -938,8 +1009,8 @@ __device__ __forceinline__ void fs_body(const DevGrid& g, const DevParams& p, in
         Cc[rr] = (k == l - 1) ? R(0) : cc;
         D[rr] = dd;
     }
-    G::sync();
-    solve_line<G, SOLVER, R>(A, B, Cc, D, pl, Rn, red);
+    tm.sync();
+    solve_line<SOLVER, R>(A, B, Cc, D, pl, Rn, red, tm);
     const R* x = B;
     const double* vel = DIR == 0 ? g.u : g.t_v;  // FSj: u = t_u here (see fsj_cell_coeffs)
     for (int c = tid; c < Rn; c += T) {
@@ -965,65 +1036,80 @@ __device__ __forceinline__ void fs_body(const DevGrid& g, const DevParams& p, in
 
 // Fused sediment sweep of one direction: as k_hydro_sweep.
 template <int DIR, int SOLVER, class R, class Lines>
-__device__ __forceinline__ void fs_sweep_loop(const Lines& lines, int half, int RB, double* gscr_d, int RG, int roww) {
+__device__ __forceinline__ void fs_sweep_loop(const Lines& lines, int half, int cap, int RB, double* gscr_d, int RG) {
     extern __shared__ double dyn_smem_d[];
     R* dyn_smem = reinterpret_cast<R*>(dyn_smem_d);
-    R* gscr = reinterpret_cast<R*>(gscr_d);
     __shared__ LineShared sgw[kWL];
-    __shared__ int s_long[kWL], s_mem[kWL], s_line[kWL];
-    __shared__ int s_nlong;
-    __shared__ R s_red[4 * kRedRows];  // reduced rows of the two-level solve
-    const int w = threadIdx.x >> 5;
+    __shared__ int s_mem[kWL], s_line[kWL];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nlines = lines.count();
     const int G = gridDim.x;
     for (int j0 = 0; (int)blockIdx.x + j0 * G < nlines; j0 += kWL) {
         const int li = blockIdx.x + (j0 + w) * G;
         LineShared& sg = sgw[w];
-        int m = 0, line = 0;
-        if (li < nlines) lines.at(li, m, line);
-        if (threadIdx.x == 0) s_nlong = 0;
-        if ((threadIdx.x & 31) == 0) {
-            s_mem[w] = m;
-            s_line[w] = line;
-        }
-        if (li < nlines) fs_setup<DIR, WarpG>(lines.grid(m), lines.params(m), line, sg);  // warp-uniform
-        __syncthreads();
-        if (li < nlines && sg.R > 0) {
-            if (sg.R > roww) {
-                if ((threadIdx.x & 31) == 0) s_long[atomicAdd(&s_nlong, 1)] = w;
-            } else {
-                const int wr = slice_rows(roww);
-                R* A = dyn_smem + w * 4 * wr;
-                fs_body<DIR, SOLVER, WarpG, R>(lines.grid(m), lines.params(m), half, line, sg, A, A + wr, A + 2 * wr,
-                                               A + 3 * wr, nullptr, SolvePlan{32, chunk_len(sg.R, 32)});
+        if (li < nlines) {  // warp-uniform
+            int m = 0, line = 0;
+            lines.at(li, m, line);
+            if (lane == 0) {
+                s_mem[w] = m;
+                s_line[w] = line;
             }
+            fs_setup<DIR, WarpG>(lines.grid(m), lines.params(m), line, sg);
+        } else if (lane == 0) {
+            sg.nseg = sg.R = 0;
         }
         __syncthreads();
-        const int nl = s_nlong;
-        for (int q = 0; q < nl; q++) {
-            const int wl = s_long[q];
-            const LineShared& sl = sgw[wl];
-            const int lm = s_mem[wl];
-            const SolvePlan pl = solve_plan(sl.R, SOLVER == 0 ? 256 : 32);
-            const bool fits = pl.t1 * pl.m <= RB;
-            const int rs = fits ? RB : RG;
-            R* A = fits ? dyn_smem : gscr + (size_t)blockIdx.x * 4 * (size_t)RG;
-            fs_body<DIR, SOLVER, BlockG, R>(lines.grid(lm), lines.params(lm), half, s_line[wl], sl, A, A + rs,
-                                            A + 2 * rs, A + 3 * rs, s_red, pl);
+        const LineShared& mine = sgw[lane & (kWL - 1)];
+        if (!__any_sync(0xffffffffu, mine.R > kRowSlice)) {  // the same in every warp
+            if (sg.R > 0) {
+                R* A = dyn_smem + w * 4 * kRowSlice;
+                fs_body<DIR, SOLVER, R>(lines.grid(s_mem[w]), lines.params(s_mem[w]), half, s_line[w], sg, A, A + kRowSlice,
+                                        A + 2 * kRowSlice, A + 3 * kRowSlice, (R*)nullptr,
+                                        SolvePlan{32, chunk_len(sg.R, 32)}, WarpTeam());
+            }
             __syncthreads();
+            continue;
+        }
+        const SolvePlan mp = solve_plan(mine.R, SOLVER == 0 ? 256 : 32);
+        const int need = 4 * mp.rows() + 4 * mp.red() + (mp.rows() > RB ? cap : 0);
+        unsigned todo = __ballot_sync(0xffffffffu, lane < kWL && mine.R > 0);
+        while (todo) {
+            TeamPick t = pick_team(todo, need, cap);
+            const bool global = t.sel == 0;  // the first line left, by the whole CTA
+            if (global) {
+                t.line = __ffs(todo) - 1;
+                t.sel = 1u << t.line;
+                t.warps = kWL;
+            }
+            const LineShared& sl = sgw[t.line];
+            const Team tm(t.first, t.warps);
+            const int pv = __shfl_sync(0xffffffffu, mp.m << 10 | mp.t1, t.line);
+            const SolvePlan pl{pv & 1023, pv >> 10};
+            const int lm = s_mem[t.line], ln = s_line[t.line];
+            if (__builtin_expect(!global, 1)) {
+                const int P = pl.rows();
+                R* A = dyn_smem + t.off;
+                fs_body<DIR, SOLVER, R>(lines.grid(lm), lines.params(lm), half, ln, sl, A, A + P, A + 2 * P, A + 3 * P,
+                                        A + 4 * P, pl, tm);
+            } else {
+                R* A = reinterpret_cast<R*>(gscr_d) + (size_t)blockIdx.x * 4 * (size_t)RG;
+                fs_body<DIR, SOLVER, R>(lines.grid(lm), lines.params(lm), half, ln, sl, A, A + RG, A + 2 * RG, A + 3 * RG,
+                                        dyn_smem, pl, tm);
+            }
+            todo &= ~t.sel;
+            __syncthreads();  // the regions and sgw are reused
         }
     }
 }
 
 template <int DIR, int SOLVER, class R>
-__global__ void __launch_bounds__(kTL, 1) k_fs_sweep(DevGrid g, DevParams p, int half, int startidx, int endidx, int RB,
-                                                  double* gscr_d, int RG, int roww) {
-    fs_sweep_loop<DIR, SOLVER, R>(OneGridLines{g, p, startidx, endidx - startidx + 1}, half, RB, gscr_d, RG, roww);
+__global__ void __launch_bounds__(kTL, 1) k_fs_sweep(DevGrid g, DevParams p, int half, int startidx, int endidx, int cap,
+                                                  int RB, double* gscr_d, int RG) {
+    fs_sweep_loop<DIR, SOLVER, R>(OneGridLines{g, p, startidx, endidx - startidx + 1}, half, cap, RB, gscr_d, RG);
 }
 template <int DIR, int SOLVER, class R>
-__global__ void __launch_bounds__(kTL, 1) k_fs_sweep_b(BatchLines bl, int half, int RB, double* gscr_d, int RG,
-                                                    int roww) {
-    fs_sweep_loop<DIR, SOLVER, R>(bl, half, RB, gscr_d, RG, roww);
+__global__ void __launch_bounds__(kTL, 1) k_fs_sweep_b(BatchLines bl, int half, int cap, int RB, double* gscr_d, int RG) {
+    fs_sweep_loop<DIR, SOLVER, R>(bl, half, cap, RB, gscr_d, RG);
 }
 
 // Largest dynamic shared memory the kernel may be given on this device.
@@ -1049,10 +1135,10 @@ cudaError_t allow_all(F* const* fs, int n, int* limit) {
     return cudaSuccess;
 }
 
-using HydroSweepFn = void(DevGrid, DevParams, int, int, int, double*, int, int);
-using FsSweepFn = void(DevGrid, DevParams, int, int, int, int, double*, int, int);
-using HydroSweepBFn = void(BatchLines, int, double*, int, int);
-using FsSweepBFn = void(BatchLines, int, int, double*, int, int);
+using HydroSweepFn = void(DevGrid, DevParams, int, int, int, int, double*, int);
+using FsSweepFn = void(DevGrid, DevParams, int, int, int, int, int, double*, int);
+using HydroSweepBFn = void(BatchLines, int, int, double*, int);
+using FsSweepBFn = void(BatchLines, int, int, int, double*, int);
 
 // [precision: 0 FP64, 1 mixed][direction][solver]
 HydroSweepFn* const kHydroSweep[2][2][2] = {
@@ -1064,6 +1150,27 @@ FsSweepFn* const kFsSweep[2][2][2] = {
     {{k_fs_sweep<0, 0, double>, k_fs_sweep<0, 1, double>}, {k_fs_sweep<1, 0, double>, k_fs_sweep<1, 1, double>}},
     {{k_fs_sweep<0, 0, float>, k_fs_sweep<0, 1, float>}, {k_fs_sweep<1, 0, float>, k_fs_sweep<1, 1, float>}}};
 
+HydroSweepBFn* const kHydroSweepB[2][2][2] = {
+    {{k_hydro_sweep_b<0, 0, double>, k_hydro_sweep_b<0, 1, double>},
+     {k_hydro_sweep_b<1, 0, double>, k_hydro_sweep_b<1, 1, double>}},
+    {{k_hydro_sweep_b<0, 0, float>, k_hydro_sweep_b<0, 1, float>},
+     {k_hydro_sweep_b<1, 0, float>, k_hydro_sweep_b<1, 1, float>}}};
+FsSweepBFn* const kFsSweepB[2][2][2] = {
+    {{k_fs_sweep_b<0, 0, double>, k_fs_sweep_b<0, 1, double>}, {k_fs_sweep_b<1, 0, double>, k_fs_sweep_b<1, 1, double>}},
+    {{k_fs_sweep_b<0, 0, float>, k_fs_sweep_b<0, 1, float>}, {k_fs_sweep_b<1, 0, float>, k_fs_sweep_b<1, 1, float>}}};
+
+}  // namespace
+
+// Values of shared memory a launch asks for: the longest line it may hold on chip, or room for
+// `n` lines side by side (the lines a CTA takes at once) of up to kRowW rows (wide) or
+// kRowSlice, whichever is more; more lines than fit are swept in rounds.
+namespace {
+int sweep_cap(const SweepPlan& sp, int fs, int n, int wide) {
+    const int one = fs ? 4 * sp.RBf + 4 * kRedRows : 4 * sp.RB + kEnds + 4 * kRedRows;
+    const int side = n * (4 * (wide ? kRowW : kRowSlice) + (fs ? 0 : kEnds));
+    const int lim = fs ? sp.lim_f : sp.lim_h;
+    return std::min(std::max(one, side), lim);
+}
 }  // namespace
 
 // Shared-memory sizes and the long-line grid of a grid of N x M cells on the current
@@ -1076,10 +1183,19 @@ cudaError_t sweep_plan(int N, int M, SweepPlan* sp, int max_rows) {
     // the bytes of the same plan
     if ((e = allow_all(&kHydroSweep[0][0][0], 8, &lim_h)) != cudaSuccess) return e;
     if ((e = allow_all(&kFsSweep[0][0][0], 8, &lim_f)) != cudaSuccess) return e;
+    // the batched kernels' static shared memory may differ: the plan fits both
+    for (int i = 0; i < 8; i++) {
+        lim_h = std::min(lim_h, max_dyn_smem((const void*)(&kHydroSweepB[0][0][0])[i]));
+        lim_f = std::min(lim_f, max_dyn_smem((const void*)(&kFsSweepB[0][0][0])[i]));
+    }
     const int L = N > M ? N : M;
-    const size_t warp_h = (size_t)kWL * kWarpHydro, warp_f = (size_t)kWL * kWarpFs;  // short-line slices
-    if ((long long)(sizeof(double) * warp_h) > lim_h || (long long)(sizeof(double) * warp_f) > lim_f)
+    // a line's region: its rows, a hydrodynamic line's segment ends, the reduced rows of a
+    // two-level solve
+    const size_t fix_h = kEnds + 4 * (size_t)kRedRows, fix_f = 4 * (size_t)kRedRows;
+    if ((long long)(sizeof(double) * (fix_h + 4 * kRowW)) > lim_h || (long long)(sizeof(double) * (fix_f + 4 * kRowW)) > lim_f)
         return cudaErrorInvalidValue;
+    sp->lim_h = lim_h / (int)sizeof(double);
+    sp->lim_f = lim_f / (int)sizeof(double);
     // every row a line can have: rows <= 2 L + 20 (solved by 32 lanes)
     {
         int rg = 0;
@@ -1091,35 +1207,33 @@ cudaError_t sweep_plan(int N, int M, SweepPlan* sp, int max_rows) {
     }
     sp->need_global = 0;
     sp->wide = 0;
-    if ((long long)(sizeof(double) * (4 * (size_t)sp->RG + kEnds)) <= lim_h) {
+    if (4 * (size_t)sp->RG + fix_h <= (size_t)sp->lim_h) {
         sp->RB = sp->RG;
     } else {  // as many rows as fit; longer lines use global scratch
-        sp->RB = (int)((lim_h / (int)sizeof(double) - kEnds) / 4);
+        sp->RB = (int)((sp->lim_h - fix_h) / 4);
         sp->need_global = 1;
     }
     if (max_rows > 0 && sp->RB > max_rows) {
         sp->RB = max_rows;
         sp->need_global = 1;
     }
-    size_t big = 4 * (size_t)sp->RB + kEnds;
-    sp->smem_lines = sizeof(double) * (big > warp_h ? big : warp_h);
     sp->RGf = 0;
     for (int t1 = 32; t1 <= 256; t1 <<= 1) {
         const int r = t1 * chunk_len(L, t1);
         if (r > sp->RGf) sp->RGf = r;
     }
-    if ((long long)(sizeof(double) * 4 * (size_t)sp->RGf) <= lim_f) {
+    if (4 * (size_t)sp->RGf + fix_f <= (size_t)sp->lim_f) {
         sp->RBf = sp->RGf;
     } else {
-        sp->RBf = (int)((lim_f / (int)sizeof(double)) / 4);
+        sp->RBf = (int)((sp->lim_f - fix_f) / 4);
         sp->need_global = 1;
     }
     if (max_rows > 0 && sp->RBf > max_rows) {
         sp->RBf = max_rows;
         sp->need_global = 1;
     }
-    big = 4 * (size_t)sp->RBf;
-    sp->smem_fs_lines = sizeof(double) * (big > warp_f ? big : warp_f);
+    sp->smem_lines = sizeof(double) * (size_t)sweep_cap(*sp, 0, kWL, 0);
+    sp->smem_fs_lines = sizeof(double) * (size_t)sweep_cap(*sp, 1, kWL, 0);
     int dev = 0, nsm = 0, occ = 0, occf = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -1146,19 +1260,22 @@ void sweep_plan_throughput(int N, int M, SweepPlan* sp) {
 }
 
 namespace {
+// Shared memory of a launch over nlines lines: the wide room where the plan asks for it (batch
+// members) and where a CTA takes more than kWL lines, so that few rounds are needed.
+int launch_cap(const SweepPlan& sp, int fs, int nlines) {
+    const int per = (nlines + sp.long_grid - 1) / sp.long_grid;
+    return sweep_cap(sp, fs, std::min(kWL, per), sp.wide || per > kWL);
+}
+
 void hydro_sweep(int dir, const DevGrid& g, const DevParams& p, const SweepPlan& sp, int startidx, int endidx,
                  int solver, double* scratch, cudaStream_t s) {
     const int nlines = endidx - startidx + 1;
     if (nlines <= 0) return;
     const int sv = solver ? 1 : 0;
-    const int roww = (sp.wide || nlines > kWL * sp.long_grid) ? kRowW : kRowShort;
-    // the long-line rows or the warps' slices, whichever is larger (a smaller request
-    // leaves more of the SM's on-chip memory to L1)
-    const size_t big = 4 * (size_t)sp.RB + kEnds, slices = (size_t)kWL * (4 * slice_rows(roww) + kEnds);
+    const int cap = launch_cap(sp, 0, nlines);
     const size_t esz = p.mixed ? sizeof(float) : sizeof(double);
-    const size_t smem = esz * (big > slices ? big : slices);
-    kHydroSweep[p.mixed ? 1 : 0][dir][sv]<<<sp.long_grid, kTL, smem, s>>>(g, p, startidx, endidx, sp.RB, scratch,
-                                                                         sp.RG, roww);
+    kHydroSweep[p.mixed ? 1 : 0][dir][sv]<<<sp.long_grid, kTL, esz * cap, s>>>(g, p, startidx, endidx, cap, sp.RB, scratch,
+                                                                              sp.RG);
     hyd_kernel_launches_add(1);
 }
 
@@ -1167,12 +1284,10 @@ void fs_sweep(int dir, const DevGrid& g, const DevParams& p, const SweepPlan& sp
     const int nlines = endidx - startidx + 1;
     if (nlines <= 0) return;
     const int sv = solver ? 1 : 0;
-    const int roww = (sp.wide || nlines > kWL * sp.long_grid) ? kRowW : kRowShortF;
-    const size_t big = 4 * (size_t)sp.RBf, slices = (size_t)kWL * 4 * slice_rows(roww);
+    const int cap = launch_cap(sp, 1, nlines);
     const size_t esz = p.mixed ? sizeof(float) : sizeof(double);
-    const size_t smem = esz * (big > slices ? big : slices);
-    kFsSweep[p.mixed ? 1 : 0][dir][sv]<<<sp.long_grid, kTL, smem, s>>>(g, p, half, startidx, endidx, sp.RBf, scratch,
-                                                                      sp.RGf, roww);
+    kFsSweep[p.mixed ? 1 : 0][dir][sv]<<<sp.long_grid, kTL, esz * cap, s>>>(g, p, half, startidx, endidx, cap, sp.RBf,
+                                                                           scratch, sp.RGf);
     hyd_kernel_launches_add(1);
 }
 }  // namespace
@@ -1211,56 +1326,20 @@ void launch_fs_sweep_i(const DevGrid& g, const DevParams& p, const SweepPlan& sp
 }
 
 // ---- batched sweeps: every member's lines in one persistent launch (the common plan of
-// the batch: rows kept in shared memory, warp tier wide)
+// the batch: the largest member's)
 void launch_sweep_batch(int dir, const BatchLines& bl, const SweepPlan& sp, int solver, int mixed, double* scratch,
                         int grid, cudaStream_t s) {
-    const int sv = solver ? 1 : 0;
-    const int roww = kRowW;
-    const size_t big = 4 * (size_t)sp.RB + kEnds, slices = (size_t)kWL * (4 * slice_rows(roww) + kEnds);
-    const size_t smem = (mixed ? sizeof(float) : sizeof(double)) * (big > slices ? big : slices);
-    if (mixed) {
-        if (dir == 0) {
-            if (sv) k_hydro_sweep_b<0, 1, float><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-            else k_hydro_sweep_b<0, 0, float><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-        } else {
-            if (sv) k_hydro_sweep_b<1, 1, float><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-            else k_hydro_sweep_b<1, 0, float><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-        }
-    } else {
-        if (dir == 0) {
-            if (sv) k_hydro_sweep_b<0, 1, double><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-            else k_hydro_sweep_b<0, 0, double><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-        } else {
-            if (sv) k_hydro_sweep_b<1, 1, double><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-            else k_hydro_sweep_b<1, 0, double><<<grid, kTL, smem, s>>>(bl, sp.RB, scratch, sp.RG, roww);
-        }
-    }
+    const int cap = sp.lim_h;
+    const size_t esz = mixed ? sizeof(float) : sizeof(double);
+    kHydroSweepB[mixed ? 1 : 0][dir][solver ? 1 : 0]<<<grid, kTL, esz * cap, s>>>(bl, cap, sp.RB, scratch, sp.RG);
     hyd_kernel_launches_add(1);
 }
 
 void launch_fs_sweep_batch(int dir, const BatchLines& bl, const SweepPlan& sp, int half, int solver, int mixed,
                            double* scratch, int grid, cudaStream_t s) {
-    const int sv = solver ? 1 : 0;
-    const int roww = kRowW;
-    const size_t big = 4 * (size_t)sp.RBf, slices = (size_t)kWL * 4 * slice_rows(roww);
-    const size_t smem = (mixed ? sizeof(float) : sizeof(double)) * (big > slices ? big : slices);
-    if (mixed) {
-        if (dir == 0) {
-            if (sv) k_fs_sweep_b<0, 1, float><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-            else k_fs_sweep_b<0, 0, float><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-        } else {
-            if (sv) k_fs_sweep_b<1, 1, float><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-            else k_fs_sweep_b<1, 0, float><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-        }
-    } else {
-        if (dir == 0) {
-            if (sv) k_fs_sweep_b<0, 1, double><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-            else k_fs_sweep_b<0, 0, double><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-        } else {
-            if (sv) k_fs_sweep_b<1, 1, double><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-            else k_fs_sweep_b<1, 0, double><<<grid, kTL, smem, s>>>(bl, half, sp.RBf, scratch, sp.RGf, roww);
-        }
-    }
+    const int cap = sp.lim_f;
+    const size_t esz = mixed ? sizeof(float) : sizeof(double);
+    kFsSweepB[mixed ? 1 : 0][dir][solver ? 1 : 0]<<<grid, kTL, esz * cap, s>>>(bl, half, cap, sp.RBf, scratch, sp.RGf);
     hyd_kernel_launches_add(1);
 }
 
@@ -1273,15 +1352,8 @@ void launch_coef_fsj_batch(const BatchRef& br, int ctas, int half, int mixed, cu
 // The batched sweeps may use all the shared memory the device allows (their row plans
 // are the largest member's).
 cudaError_t batch_sweep_setup() {
-    HydroSweepBFn* const hb[8] = {k_hydro_sweep_b<0, 0, double>, k_hydro_sweep_b<0, 1, double>,
-                                 k_hydro_sweep_b<1, 0, double>, k_hydro_sweep_b<1, 1, double>,
-                                 k_hydro_sweep_b<0, 0, float>,  k_hydro_sweep_b<0, 1, float>,
-                                 k_hydro_sweep_b<1, 0, float>,  k_hydro_sweep_b<1, 1, float>};
-    FsSweepBFn* const fb[8] = {k_fs_sweep_b<0, 0, double>, k_fs_sweep_b<0, 1, double>, k_fs_sweep_b<1, 0, double>,
-                              k_fs_sweep_b<1, 1, double>, k_fs_sweep_b<0, 0, float>,  k_fs_sweep_b<0, 1, float>,
-                              k_fs_sweep_b<1, 0, float>,  k_fs_sweep_b<1, 1, float>};
     int lim;
-    cudaError_t e = allow_all(hb, 8, &lim);
-    if (e == cudaSuccess) e = allow_all(fb, 8, &lim);
+    cudaError_t e = allow_all(&kHydroSweepB[0][0][0], 8, &lim);
+    if (e == cudaSuccess) e = allow_all(&kFsSweepB[0][0][0], 8, &lim);
     return e;
 }

@@ -225,7 +225,7 @@ class Simulation:
         _check(self.lib.hyd_mirror_close(self.h))
 
     def set_sweep_shape(self, ctas, wide):
-        """Sweep CTAs (0: one per SM) and whether warps take every line up to 288 rows."""
+        """Sweep CTAs (0: one per SM) and whether a CTA holds 16 lines of up to 288 rows at once."""
         _check(self.lib.hyd_set_sweep_shape(self.h, int(ctas), int(wide)))
 
     def sweep_shape(self):

@@ -2,18 +2,19 @@
 
 A batch's members run side by side on one GPU, so the best sweep shape depends on the
 whole batch, not on one reach: how many persistent CTAs each member's sweeps take (a
-member's CTAs hold whole SMs while they run) and whether warps sweep every line of up to
-288 rows or only those of up to 96 (the rest by the whole CTA, one after another).  The
+member's CTAs hold whole SMs while they run) and whether a CTA asks for the shared memory to
+sweep 16 lines of up to 288 rows side by side, or only of up to 96 (more of the SM's on-chip
+memory left to L1).  The
 tuner steps the batch under each candidate policy for a few steps, times them, and keeps
 the fastest.  The tuning steps are ordinary steps of the simulation (every shape gives
-the same results up to rounding, within the parity tolerance), so nothing is saved or
+the same results), so nothing is saved or
 restored.
 
     tune_batch(batch, candidates, steps) -> (best policy, {policy: seconds per step})
 
 A policy (d, wide) steps every member on its own stream and graph and gives member k
 ceil((max(N_k, M_k) + 3) / d) sweep CTAs (d lines per CTA: one per warp at d = 16) and
-the warp-tier choice `wide`.  The policy FUSED steps the batch by batched launches
+the shared-memory choice `wide`.  The policy FUSED steps the batch by batched launches
 (hyd_batch_set_fused: every phase one launch for all members, the lines of all members
 in one persistent sweep of one CTA per SM).  Which is faster depends on the batch: the
 batched launches wait, phase by phase, for the member with the longest chain, while the

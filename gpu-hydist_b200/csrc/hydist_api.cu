@@ -1118,9 +1118,21 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
         launch_budget_half(g, p, 1, s->side2);
         cudaEventRecord(s->ev_bjoin, s->side2);
     }
-    { PHASE(PH_SMOOTH); launch_smooth(g, p, 1, s->scratch_u, fh, 0, 0, fh, st); }
-    std::swap(g.t_u, s->scratch_u);
-    { PHASE(PH_EXPL_V); launch_explicit_v(g, p, s->thr_r, st); }
+    // span-limited steps whose segment tables follow the mask take the explicit momentum cell
+    // by cell, on smaller grids (msm) with the smoothing before it in the same pass; a step that
+    // owes a rescan of every line (tables set by the caller) or whole-grid passes takes it from
+    // the tables, line by line, and so does v on larger grids, where its rows are contiguous
+    // and a CTA per row is the faster form (4096 x 2048: 30 against 38 us)
+    const int mom = !fh && !force, msm = mom && !s->plan.wide && mom_smooths(g);
+    if (msm) {
+        PHASE(PH_EXPL_V);
+        launch_mom(g, p, 1, 1, s->scratch_u, st);
+        std::swap(g.t_u, s->scratch_u);
+    } else {
+        { PHASE(PH_SMOOTH); launch_smooth(g, p, 1, s->scratch_u, fh, 0, 0, fh, st); }
+        std::swap(g.t_u, s->scratch_u);
+        { PHASE(PH_EXPL_V); launch_explicit_v(g, p, s->thr_r, st); }
+    }
     { PHASE(PH_SMOOTH); launch_smooth(g, p, 0, s->scratch_v, fh, 0, 0, 0, st); }
     std::swap(g.t_v, s->scratch_v);
     if (force) launch_mark_all_cols(g, st);
@@ -1172,10 +1184,19 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
         launch_budget_half(g, p, 0, s->side2);
         cudaEventRecord(s->ev_bjoin, s->side2);
     }
-    { PHASE(PH_SMOOTH); launch_smooth(g, p, 0, s->scratch_v, fh, 0, 0, fh, st); }
-    std::swap(g.t_v, s->scratch_v);
-    { PHASE(PH_COEF_EU); launch_coef_eu(g, p, st); }
-    { PHASE(PH_EXPL_U); launch_explicit_u(g, p, s->thr_c, st); }
+    if (!msm) {
+        PHASE(PH_SMOOTH);
+        launch_smooth(g, p, 0, s->scratch_v, fh, 0, 0, fh, st);
+        std::swap(g.t_v, s->scratch_v);
+    }
+    if (mom) {
+        PHASE(PH_EXPL_U);
+        launch_mom(g, p, 0, msm, s->scratch_v, st);
+        if (msm) std::swap(g.t_v, s->scratch_v);
+    } else {
+        { PHASE(PH_COEF_EU); launch_coef_eu(g, p, st); }
+        { PHASE(PH_EXPL_U); launch_explicit_u(g, p, s->thr_c, st); }
+    }
     if (overlap) cudaStreamWaitEvent(st, s->ev_join, 0);
     { PHASE(PH_SMOOTH); launch_smooth(g, p, 1, s->scratch_u, fh, 1, overlap, 0, st); }
     std::swap(g.t_u, s->scratch_u);
@@ -1804,7 +1825,7 @@ int hyd_launch_count(hyd_handle h, long long* count) {
 // ---- batches of independent reaches (one persistent handle per member)
 
 // Phases of a batched step with their own per-member CTA counts.
-enum BatchPhase { BP_CB, BP_SM_BUD, BP_SM, BP_SM_FSB, BP_EV, BP_CEU, BP_EU, BP_RR, BP_RC, BP_PF, BP_FSJC, BP_UFS,
+enum BatchPhase { BP_CB, BP_SM_BUD, BP_SM, BP_SM_FSB, BP_EV, BP_RR, BP_RC, BP_PF, BP_FSJC, BP_UFS,
                   BP_COUNT };
 // Line lists of the batched sweeps.
 enum BatchLineSet { BL_UZ, BL_VZ, BL_FSJ, BL_FSI, BL_COUNT };
@@ -1827,7 +1848,7 @@ struct BatchFused {
     double* gscr = nullptr;     // sweep rows of lines too long for shared memory (if any)
     double* gscr_fs = nullptr;  // the same for the sediment sweep beside the main chain
     int thr_r = 64, thr_c = 64;
-    size_t sm_ev = 0, sm_eu = 0, sm_rr = 0, sm_rc = 0, sm_pf = 0;
+    size_t sm_ev = 0, sm_rr = 0, sm_rc = 0, sm_pf = 0;
     cudaStream_t st = nullptr, side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
     std::vector<cudaEvent_t> mev;  // per member: its stream's work before a batched run
@@ -1979,8 +2000,6 @@ int fused_build(HydBatch* b) {
         counts[BP_SM].push_back(rw);
         counts[BP_SM_FSB].push_back(rw + 1);
         counts[BP_EV].push_back(N - 1);
-        counts[BP_CEU].push_back(((N - 2) * 32 + 255) / 256);
-        counts[BP_EU].push_back(M - 1);
         counts[BP_RR].push_back(N);
         counts[BP_RC].push_back(M);
         counts[BP_PF].push_back(row_warp_ctas(g0, N + 1) + 32 + 8);
@@ -1998,10 +2017,9 @@ int fused_build(HydBatch* b) {
         Mmax = std::max(Mmax, M);
         f.thr_r = std::max(f.thr_r, s->thr_r);
         f.thr_c = std::max(f.thr_c, s->thr_c);
-        size_t ev, eu, rr, rc, pf;
-        line_smem(N, M, &ev, &eu, &rr, &rc, &pf);
+        size_t ev, rr, rc, pf;
+        line_smem(N, M, &ev, &rr, &rc, &pf);
         f.sm_ev = std::max(f.sm_ev, ev);
-        f.sm_eu = std::max(f.sm_eu, eu);
         f.sm_rr = std::max(f.sm_rr, rr);
         f.sm_rc = std::max(f.sm_rc, rc);
         f.sm_pf = std::max(f.sm_pf, pf);
@@ -2060,7 +2078,7 @@ int fused_build(HydBatch* b) {
         CUDA_TRY(cudaMalloc(&f.gscr_fs, rows * f.grid * sizeof(double)));
     }
     CUDA_TRY(batch_sweep_setup());
-    CUDA_TRY(batch_grid_setup(f.sm_ev, f.sm_eu, f.sm_rr, f.sm_rc, f.sm_pf));
+    CUDA_TRY(batch_grid_setup(f.sm_ev, f.sm_rr, f.sm_rc, f.sm_pf));
     int prio_lo = 0, prio_hi = 0;
     cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
     CUDA_TRY(cudaStreamCreateWithPriority(&f.st, cudaStreamNonBlocking, prio_hi));
@@ -2104,8 +2122,7 @@ void fused_launch_step(HydBatch* b, int sed1, int sed2, int bed) {
     launch_coef_bnd_batch(BR(2, BP_CB), f.ctas[BP_CB], 1, sed1 ? 1 : 3, mx, st);
     launch_sweep_batch(1, BL(2, BL_VZ), f.plan, f.solver, mx, f.gscr, f.grid, st);
     launch_smooth_batch(BR(2, BP_SM_BUD), f.ctas[BP_SM_BUD], 0, f.outs[2], 0, 0, 1, st);
-    launch_coef_eu_batch(BR(1, BP_CEU), f.ctas[BP_CEU], mx, st);
-    launch_explicit_u_batch(BR(1, BP_EU), f.ctas[BP_EU], f.thr_c, f.sm_eu, mx, st);
+    launch_mom_u_batch(BR(1, BP_SM), f.ctas[BP_SM], mx, st);
     if (sed1) cudaStreamWaitEvent(st, f.join, 0);
     launch_smooth_batch(BR(1, sed1 ? BP_SM_FSB : BP_SM), f.ctas[sed1 ? BP_SM_FSB : BP_SM], 1, f.outs[3], 1, sed1, 0,
                         st);

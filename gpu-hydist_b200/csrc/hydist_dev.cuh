@@ -356,6 +356,10 @@ void launch_budget_half(const DevGrid& g, const DevParams& p, int isU, cudaStrea
 void launch_smooth(const DevGrid& g, const DevParams& p, int isU, double* out, int full, int bytes, int fs_bnd,
                    int budget, cudaStream_t s);
 void launch_widen_spans(const DevGrid& g, cudaStream_t s);
+// Span-limited steps: one component's explicit momentum (dir 1: v, dir 0: u), with `smooth` also
+// the smoothing of the other, swept component into out (else it is smoothed already).
+int mom_smooths(const DevGrid& g);
+void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, double* out, cudaStream_t s);
 void launch_explicit_v(const DevGrid& g, const DevParams& p, int threads, cudaStream_t s);
 void launch_explicit_u(const DevGrid& g, const DevParams& p, int threads, cudaStream_t s);
 void launch_coef_eu(const DevGrid& g, const DevParams& p, cudaStream_t s);
@@ -410,8 +414,7 @@ void launch_coef_bnd_batch(const BatchRef& br, int ctas, int half, int writes, i
 void launch_smooth_batch(const BatchRef& br, int ctas, int isU, double* const* outs, int bytes, int fs_bnd, int budget,
                          cudaStream_t s);
 void launch_explicit_v_batch(const BatchRef& br, int ctas, int threads, size_t smem, int mixed, cudaStream_t s);
-void launch_coef_eu_batch(const BatchRef& br, int ctas, int mixed, cudaStream_t s);
-void launch_explicit_u_batch(const BatchRef& br, int ctas, int threads, size_t smem, int mixed, cudaStream_t s);
+void launch_mom_u_batch(const BatchRef& br, int ctas, int mixed, cudaStream_t s);
 void launch_reset_batch(const BatchRef& br, int ctas, int rows, int threads, size_t smem, cudaStream_t s);
 void launch_post_fused_batch(const BatchRef& br, int ctas, int rows, int vth, int mixed, size_t smem, cudaStream_t s);
 void launch_update_fs_batch(const BatchRef& br, int ctas, cudaStream_t s);
@@ -420,6 +423,6 @@ void launch_sweep_batch(int dir, const BatchLines& bl, const SweepPlan& sp, int 
                         int grid, cudaStream_t s);
 void launch_fs_sweep_batch(int dir, const BatchLines& bl, const SweepPlan& sp, int half, int solver, int mixed,
                            double* scratch, int grid, cudaStream_t s);
-cudaError_t batch_grid_setup(size_t smem_ev, size_t smem_eu, size_t smem_rr, size_t smem_rc, size_t smem_pf);
+cudaError_t batch_grid_setup(size_t smem_ev, size_t smem_rr, size_t smem_rc, size_t smem_pf);
 cudaError_t batch_sweep_setup();
-void line_smem(int N, int M, size_t* ev, size_t* eu, size_t* rr, size_t* rc, size_t* pf);
+void line_smem(int N, int M, size_t* ev, size_t* rr, size_t* rc, size_t* pf);

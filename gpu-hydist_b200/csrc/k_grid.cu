@@ -523,10 +523,8 @@ __global__ void __launch_bounds__(256) k_coef_bnd_b(BatchRef br, int writes) {
 // the interior, a copy elsewhere.  isU smooths t_u (neighbours along i, wet check along j).
 // A nonzero velocity outside the row's extended span is reported in *g.span_wide (the
 // spans then cannot bound the smoothing).
-__device__ __forceinline__ void smooth_cell(const DevGrid& g, const DevParams& p, int isU, double* __restrict__ out,
-                                            int i, int j, bool check_span) {
+__device__ __forceinline__ double smooth_value(const DevGrid& g, const DevParams& p, int isU, int i, int j) {
     const int N = g.N, M = g.M, P = g.P;
-    if (i >= N + 3 || j >= M + 3) return;
     const double* val = isU ? g.t_u : g.t_v;
     const int gp = i * P + j;
     const bool inner = !(i > N || j > M || i < 2 || j < 2);
@@ -545,7 +543,6 @@ __device__ __forceinline__ void smooth_cell(const DevGrid& g, const DevParams& p
         kfp = g.khouot[gp + far_d];
     }
     double r = v0;
-    if (check_span && v0 != 0 && (j < g.elo[i] || j > g.ehi[i])) *g.span_wide = 1;
     if (inner && v0 != 0) {
         int count = 2;
         double nb = vcm + vcp;
@@ -559,7 +556,15 @@ __device__ __forceinline__ void smooth_cell(const DevGrid& g, const DevParams& p
         }
         r = v0 * p.heso + (1 - p.heso) * nb / count;
     }
-    out[gp] = r;
+    return r;
+}
+
+__device__ __forceinline__ void smooth_cell(const DevGrid& g, const DevParams& p, int isU, double* __restrict__ out,
+                                            int i, int j, bool check_span) {
+    if (i >= g.N + 3 || j >= g.M + 3) return;
+    const int gp = i * g.P + j;
+    if (check_span && (isU ? g.t_u : g.t_v)[gp] != 0 && (j < g.elo[i] || j > g.ehi[i])) *g.span_wide = 1;
+    out[gp] = smooth_value(g, p, isU, i, j);
 }
 
 // The column-major reset byte of cell (i, j) for the column resets that follow (k_reset
@@ -844,11 +849,11 @@ __global__ void k_smooth_span_b(BatchRef br, int isU, double* const* outs) {
 // ----------------------------------------------------------- explicit momentum
 
 // vSolver (UVZSolver_multithread.cu:727-768) for one cell in the arithmetic type R: the new
-// v velocity.
-template <class R>
-__device__ __forceinline__ R ev_cell(const DevGrid& g, const DevParams& p, int row, int col) {
+// v velocity; tu(row, col): the swept and smoothed u.
+template <class R, class TU>
+__device__ __forceinline__ R ev_cell(const DevGrid& g, const DevParams& p, int row, int col, TU tu) {
     const int o = g.P;
-    const double *u = g.u, *v = g.v, *z = g.z, *t_u = g.t_u, *H = g.H_moi;
+    const double *u = g.u, *v = g.v, *z = g.z, *H = g.H_moi;
     auto L = [](const double* a, int q) { return R(a[q]); };
     R pp, q, tmp;
     q = 0;
@@ -856,7 +861,7 @@ __device__ __forceinline__ R ev_cell(const DevGrid& g, const DevParams& p, int r
     tmp = 0;
     const R v0 = L(v, row * o + col);
     const R utb = (L(u, (row - 1) * o + col) + L(u, row * o + col) + L(u, (row - 1) * o + col + 1) + L(u, row * o + col + 1)) * R(0.25);
-    const R t_utb = (L(t_u, (row - 1) * o + col) + L(t_u, row * o + col) + L(t_u, (row - 1) * o + col + 1) + L(t_u, row * o + col + 1)) * R(0.25);
+    const R t_utb = (R(tu(row - 1, col)) + R(tu(row, col)) + R(tu(row - 1, col + 1)) + R(tu(row, col + 1))) * R(0.25);
     pp = (L(v, row * o + col + 1) - L(v, row * o + col - 1)) / R(p.dY2);
     pp = R(p.HaiChiadT) + pp + L(g.Ky1, row * o + col) * sqrt(utb * utb + v0 * v0) / L(g.Htdv, row * o + col);
     // the neighbours the branches take, loaded before the depth tests (one round trip)
@@ -928,7 +933,7 @@ __device__ __forceinline__ void explicit_v_body(const DevGrid& g, const DevParam
         int k = 0;
         while (k + 1 < nseg && s_off[k + 1] <= c) k++;
         const int col = s_first[k] + (c - s_off[k]);
-        const double tv = ev_cell<R>(g, p, row, col);
+        const double tv = ev_cell<R>(g, p, row, col, [&](int r, int c) { return g.t_u[r * P + c]; });
         g.t_v[row * P + col] = tv;
         sv[col - k0] = tv;
     }
@@ -960,12 +965,12 @@ __global__ void k_explicit_v_b(BatchRef br) {
 }
 
 // uSolver (UVZSolver_multithread.cu:773-815) for one cell in the arithmetic type R: the new
-// u velocity.  Cell-local, so it is computed for every wet cell by a row-major kernel and
-// stored column-major.
-template <class R>
-__device__ __forceinline__ R eu_cell(const DevGrid& g, const DevParams& p, int row, int col) {
+// u velocity; tv(row, col): the swept and smoothed v.  Cell-local; whole-grid passes compute it
+// for every wet cell by a row-major kernel and store it column-major (k_coef_eu).
+template <class R, class TV>
+__device__ __forceinline__ R eu_cell(const DevGrid& g, const DevParams& p, int row, int col, TV tv) {
     const int P = g.P;
-    const double *u = g.u, *v = g.v, *z = g.z, *t_v = g.t_v, *H = g.H_moi;
+    const double *u = g.u, *v = g.v, *z = g.z, *H = g.H_moi;
     auto L = [](const double* a, int q) { return R(a[q]); };
     const int o = P;
     R pp, q, tmp;
@@ -974,7 +979,7 @@ __device__ __forceinline__ R eu_cell(const DevGrid& g, const DevParams& p, int r
     tmp = 0;
     const R u0 = L(u, row * o + col);
     const R vtb = (L(v, row * o + col - 1) + L(v, row * o + col) + L(v, (row + 1) * o + col - 1) + L(v, (row + 1) * o + col)) * R(0.25);
-    const R t_vtb = (L(t_v, row * o + col - 1) + L(t_v, row * o + col) + L(t_v, (row + 1) * o + col - 1) + L(t_v, (row + 1) * o + col)) * R(0.25);
+    const R t_vtb = (R(tv(row, col - 1)) + R(tv(row, col)) + R(tv(row + 1, col - 1)) + R(tv(row + 1, col))) * R(0.25);
     pp = (L(u, (row + 1) * o + col) - L(u, (row - 1) * o + col)) / R(p.dX2);
     pp = (R(p.HaiChiadT) + pp + L(g.Kx1, row * o + col) * sqrt(vtb * vtb + u0 * u0) / L(g.Htdu, row * o + col));
     // as in ev_cell: the branches' neighbours loaded first
@@ -1012,13 +1017,14 @@ constexpr int kEuSlot = 4;
 // the row's span; written column-major (g.colT array kEuSlot), with TILE through a tile.
 template <int TILE, class R>
 __device__ __forceinline__ void coef_eu_body(const DevGrid& g, const DevParams& p, int bx) {
+    const auto tv = [&](int r, int c) { return g.t_v[r * g.P + c]; };
     if constexpr (!TILE) {
         const int i = 2 + ((bx * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
         if (i > g.N - 1) return;
         const int lo = max(g.rlo[i], 2), hi = min(g.rhi[i], g.M);
         for (int j = lo + lane; j <= hi; j += 32) {
             if (g.khouot[i * g.P + j] != 0) continue;
-            colTr<R>(g, kEuSlot)[(size_t)j * g.LT + i] = eu_cell<R>(g, p, i, j);
+            colTr<R>(g, kEuSlot)[(size_t)j * g.LT + i] = eu_cell<R>(g, p, i, j, tv);
         }
     } else {
         R* const dst[1] = {colTr<R>(g, kEuSlot)};
@@ -1026,7 +1032,7 @@ __device__ __forceinline__ void coef_eu_body(const DevGrid& g, const DevParams& 
             g, 2 + kTileRows * bx, g.N - 1, 2, g.M,
             [&](int i, int j, R* v) {
                 if (g.khouot[i * g.P + j] != 0) return false;
-                v[0] = eu_cell<R>(g, p, i, j);
+                v[0] = eu_cell<R>(g, p, i, j, tv);
                 return true;
             },
             dst);
@@ -1037,12 +1043,6 @@ template <int TILE, class R>
 __global__ void __launch_bounds__(256) k_coef_eu(DevGrid g, DevParams p) {
     coef_eu_body<TILE, R>(g, p, blockIdx.x);
 }
-template <int TILE, class R>
-__global__ void __launch_bounds__(256) k_coef_eu_b(BatchRef br) {
-    const BatchMember bm(br);
-    coef_eu_body<TILE, R>(bm.g, bm.p, bm.bx);
-}
-
 // solveU/uSolver (UVZSolver_multithread.cu:947-968, 773-815) on column j from the values
 // k_coef_eu stored, then update_margin_elem_U (970-1006).
 template <class R>
@@ -1110,10 +1110,114 @@ template <class R>
 __global__ void k_explicit_u(DevGrid g, DevParams p) {
     explicit_u_body<R>(g, p, blockIdx.x);
 }
+// The explicit momentum of one component over the extended spans, row-major, a thread per cell
+// (span-limited steps).  DIR 1: v (solveV and update_margin_elem_V of every row); DIR 0: u
+// (solveU and update_margin_elem_U of every column).  SMOOTH: the other, swept component is
+// smoothed into out in the same pass (DIR 1: t_u, DIR 0: t_v); every cell smooths its own
+// velocity and, where it is stepped, the three neighbours' that the step reads, again.
+//
+// A line's segments are the runs of wet cells in [2, L] that do not start at L - 1 or L, so a
+// cell's part follows from the mask around it: cells first..last-1 are stepped; the face
+// before the first and the last cell's get 0 where the line ends at a wall, and the
+// extrapolation from the two stepped cells next to them where it ends at an open edge of the
+// grid (only a segment with first == 2 or last == L can; one with last == L has at least three
+// cells, one with first == 2 and fewer than three reads the velocity that stood there).
+// Against the cell values stored column-major and a CTA per line that staged the line and
+// stepped its ends serially (kept for whole-grid passes and caller-set tables): u of a 4096 x
+// 2048 reach 29 + 25 -> 37 us.  Whether the smoothing joins it: mom_smooths.
+template <int DIR, int SMOOTH, class R>
+__device__ __forceinline__ void mom_cell(const DevGrid& g, const DevParams& p, double* __restrict__ out, int i, int j) {
+    const int P = g.P, gp = i * P + j;
+    const double* swept = DIR == 1 ? g.t_u : g.t_v;
+    double own = 0.0;
+    if (SMOOTH) {
+        own = smooth_value(g, p, DIR, i, j);
+        out[gp] = own;
+    }
+    auto sm = [&](int r, int c) {
+        if (!SMOOTH) return swept[r * P + c];
+        return r == i && c == j ? own : smooth_value(g, p, DIR, r, c);
+    };
+    const int along = DIR == 1 ? 1 : P;          // to the next cell of the line
+    const int L = DIR == 1 ? g.M : g.N;          // the line's last cell
+    const int k = DIR == 1 ? j : i;              // this cell's place on the line
+    const int line = DIR == 1 ? i : j;
+    if (line < 2 || line > (DIR == 1 ? g.N : g.M) || k < 1 || k > L) return;
+    double* t = DIR == 1 ? g.t_v : g.t_u;
+    // the mask two cells back to one ahead; 1 beyond the cells a segment may hold
+    const int* kh = g.khouot;
+    const int w0 = k >= 2 ? kh[gp] : 1, wp = k < L ? kh[gp + along] : 1, wm = k >= 3 ? kh[gp - along] : 1,
+              wm2 = k >= 4 ? kh[gp - 2 * along] : 1;
+    auto open_edge = [&](int f) -> bool {  // f: the face 1 or L; whether the line is open there
+        const double* h = g.h;
+        if (DIR == 1) return !(fabs((h[i * P + f] + h[(i - 1) * P + f]) * 0.5 - p.NANGDAY) < kEpsRef);
+        return !(fabs(h[f * P + j] + h[f * P + j - 1]) * 0.5 - p.NANGDAY < kEpsRef);
+    };
+    // the cells k0, k1 of the line whose stepped velocities s0, s1 this cell takes (0: none)
+    int k0 = 0, k1 = 0;
+    bool put = false, first = false;
+    if (w0 == 0) {
+        // the run starts at L - 2 or before
+        if (!(k <= L - 2 || (k == L - 1 ? wm == 0 : (wm == 0 && wm2 == 0)))) return;
+        if (wp == 0) {
+            put = true;
+            k0 = k;
+        } else if (k < L) {
+            // the last cell, a wall after it; of a segment [2, 2] or [2, 3] written by the thread
+            // of the face before it, which may have to read it first
+            put = !(k == 2 || (k == 3 && wm == 0));
+        } else {
+            put = true;
+            if (open_edge(L)) k0 = L - 1, k1 = L - 2;
+        }
+    } else if (wp == 0 && k + 1 <= L - 2) {  // the face before a segment's first cell
+        put = true;
+        first = k == 1;
+    }
+    bool w3 = false, w4 = false, open = false;
+    if (first) {
+        w3 = kh[gp + 2 * along] == 0;  // cells 3 and 4 in the segment (L >= 6)
+        w4 = w3 && kh[gp + 3 * along] == 0;
+        open = open_edge(1);
+        if (open) k0 = w3 ? 2 : 0, k1 = w4 ? 3 : 0;
+    }
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 1
+    for (int e = 0; e < 2; e++) {  // one copy of the step's code; the second turn only at open edges
+        const int kk = e == 0 ? k0 : k1;
+        if (kk == 0) continue;
+        const double v = DIR == 1 ? (double)ev_cell<R>(g, p, i, kk, sm) : (double)eu_cell<R>(g, p, kk, j, sm);
+        if (e == 0) s0 = v;
+        else s1 = v;
+    }
+    if (!put) return;
+    if (first) {
+        const double a = w3 ? s0 : t[gp + along], b = w4 ? s1 : t[gp + 2 * along];
+        t[gp] = open ? 2 * a - b : 0.0;
+        if (!w3) t[gp + along] = 0.0;
+        else if (!w4) t[gp + 2 * along] = 0.0;
+    } else {
+        t[gp] = k1 ? 2 * s0 - s1 : s0;
+    }
+}
+
+template <int DIR, int SMOOTH, class R>
+__device__ __forceinline__ void mom_span_body(const DevGrid& g, const DevParams& p, double* __restrict__ out, int bx) {
+    const RowLane rl(g, 0, bx);
+    const int i = rl.i;
+    if (i > g.N + 2) return;
+    for (int j = g.elo[i] + rl.off; j <= g.ehi[i]; j += rl.stride) mom_cell<DIR, SMOOTH, R>(g, p, out, i, j);
+}
+
+template <int DIR, int SMOOTH, class R>
+__global__ void __launch_bounds__(256) k_mom_span(DevGrid g, DevParams p, double* __restrict__ out) {
+    mom_span_body<DIR, SMOOTH, R>(g, p, out, blockIdx.x);
+}
+// u of every member (v is already smoothed)
 template <class R>
-__global__ void k_explicit_u_b(BatchRef br) {
+__global__ void __launch_bounds__(256) k_mom_u_b(BatchRef br) {
     const BatchMember bm(br);
-    explicit_u_body<R>(bm.g, bm.p, bm.bx);
+    mom_span_body<0, 0, R>(bm.g, bm.p, nullptr, bm.bx);
 }
 
 // --------------------------------------------------------------- wet/dry resets
@@ -2490,6 +2594,21 @@ void launch_explicit_u(const DevGrid& g, const DevParams& p, int threads, cudaSt
     hyd_kernel_launches_add(1);
 }
 
+// Whether the smoothing joins the explicit momentum's launch: while the CTAs are about a wave
+// of the device, a launch saved is worth the neighbours smoothed again (a 1048 x 980 reach, 263
+// CTAs: 88 -> 85 us a step; 1531 x 777, 383 CTAs: 95 -> 92); beyond that the arithmetic is not
+// hidden any more (2048 x 2048, 1282 CTAs: 222 us joined, 205 apart), nor where reaches share
+// the device (the callers leave it apart there: 16 reaches 297 us joined, 284 apart).
+int mom_smooths(const DevGrid& g) { return row_warps_blocks(g, g.N + 3) <= 4 * scan_grid(); }
+
+void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, double* out, cudaStream_t s) {
+    void (*const k[2][2][2])(DevGrid, DevParams, double*) = {
+        {{k_mom_span<0, 0, double>, k_mom_span<0, 0, float>}, {k_mom_span<0, 1, double>, k_mom_span<0, 1, float>}},
+        {{k_mom_span<1, 0, double>, k_mom_span<1, 0, float>}, {k_mom_span<1, 1, double>, k_mom_span<1, 1, float>}}};
+    k[dir ? 1 : 0][smooth ? 1 : 0][p.mixed ? 1 : 0]<<<row_warps_blocks(g, g.N + 3), 256, 0, s>>>(g, p, out);
+    hyd_kernel_launches_add(1);
+}
+
 void launch_reset_rows(const DevGrid& g, const DevParams& p, int force, int threads, cudaStream_t s) {
     k_reset<1><<<g.N, threads, reset_smem(g.M), s>>>(g, p, force);
     hyd_kernel_launches_add(1);
@@ -2665,15 +2784,9 @@ void launch_explicit_v_batch(const BatchRef& br, int ctas, int threads, size_t s
     hyd_kernel_launches_add(1);
 }
 
-void launch_coef_eu_batch(const BatchRef& br, int ctas, int mixed, cudaStream_t s) {
-    if (mixed) k_coef_eu_b<0, float><<<ctas, 256, 0, s>>>(br);
-    else k_coef_eu_b<0, double><<<ctas, 256, 0, s>>>(br);
-    hyd_kernel_launches_add(1);
-}
-
-void launch_explicit_u_batch(const BatchRef& br, int ctas, int threads, size_t smem, int mixed, cudaStream_t s) {
-    if (mixed) k_explicit_u_b<float><<<ctas, threads, smem, s>>>(br);
-    else k_explicit_u_b<double><<<ctas, threads, smem, s>>>(br);
+void launch_mom_u_batch(const BatchRef& br, int ctas, int mixed, cudaStream_t s) {
+    if (mixed) k_mom_u_b<float><<<ctas, 256, 0, s>>>(br);
+    else k_mom_u_b<double><<<ctas, 256, 0, s>>>(br);
     hyd_kernel_launches_add(1);
 }
 
@@ -2704,7 +2817,7 @@ void launch_update_fs_batch(const BatchRef& br, int ctas, cudaStream_t s) {
 
 // Opt the batched kernels that stage a line in shared memory into `bytes` of it (the
 // largest any member needs).
-cudaError_t batch_grid_setup(size_t smem_ev, size_t smem_eu, size_t smem_rr, size_t smem_rc, size_t smem_pf) {
+cudaError_t batch_grid_setup(size_t smem_ev, size_t smem_rr, size_t smem_rc, size_t smem_pf) {
     cudaError_t e;
     const void* pf[] = {(const void*)k_post_fused_b<0, 0, double>, (const void*)k_post_fused_b<0, 1, double>,
                         (const void*)k_post_fused_b<1, 0, double>, (const void*)k_post_fused_b<1, 1, double>,
@@ -2713,21 +2826,18 @@ cudaError_t batch_grid_setup(size_t smem_ev, size_t smem_eu, size_t smem_rr, siz
         if ((e = allow_smem(f, smem_pf)) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_explicit_v_b<double>, smem_ev)) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_explicit_v_b<float>, smem_ev)) != cudaSuccess) return e;
-    if ((e = allow_smem((const void*)k_explicit_u_b<double>, smem_eu)) != cudaSuccess) return e;
-    if ((e = allow_smem((const void*)k_explicit_u_b<float>, smem_eu)) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_reset_b<1>, smem_rr)) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_reset_b<0>, smem_rc)) != cudaSuccess) return e;
     return cudaSuccess;
 }
 
-// Shared memory the line kernels of one grid need (k_explicit_v / _u, k_reset rows /
+// Shared memory the batched line kernels of one grid need (k_explicit_v, k_reset rows /
 // columns, k_post_fused).
-void line_smem(int N, int M, size_t* ev, size_t* eu, size_t* rr, size_t* rc, size_t* pf) {
+void line_smem(int N, int M, size_t* ev, size_t* rr, size_t* rc, size_t* pf) {
     DevGrid g{};
     g.N = N;
     g.M = M;
     *ev = sizeof(double) * (M + 3);
-    *eu = sizeof(double) * (N + 3);
     *rr = reset_smem(M);
     *rc = reset_smem(N);
     *pf = scan_smem(g);

@@ -1896,10 +1896,12 @@ int hyd_batch_create(int count, const HydCaseParams* params, const int* dims, in
             delete b;
             return fail(rc, msg);
         }
-        // the members run side by side: sweeps sized by their lines, not the device
-        sweep_plan_throughput(h->N, h->M, &h->plan);
         b->members.push_back(h);
     }
+    // the members run side by side: sweeps sized by the batch's lines, not the device
+    std::vector<SweepPlan*> plans;
+    for (hyd_handle h : b->members) plans.push_back(&h->plan);
+    sweep_plan_throughput(dims, plans.data(), count);
     *out = b;
     return HYD_OK;
 }

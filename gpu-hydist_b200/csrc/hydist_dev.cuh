@@ -338,10 +338,13 @@ struct SweepPlan {
 };
 // max_rows > 0: at most that many rows of a long line in shared memory (0: as many as fit)
 cudaError_t sweep_plan(int N, int M, SweepPlan* sp, int max_rows);
-// Throughput sizing for reaches that share the device with others: as many sweep CTAs as
-// give every line of the longer direction its own warp in one pass, instead of one CTA per
-// SM, and shared memory for 16 medium lines at once.
-void sweep_plan_throughput(int N, int M, SweepPlan* sp);
+// Throughput sizing of a batch's reaches, which share the device (dims: N, M of each): sweep
+// CTAs of `per` groups of 16 lines, and shared memory for 16 medium lines at once.  A sweep CTA
+// holds a whole SM, so `per` is the number, at most 4, that makes all members' CTAs together
+// about one per SM: 3 or 4 small reaches keep a line per warp (129 us a step against 150 with
+// per = 3), 16 take per = 3 (288 -> 263), 32 per = 4 (603 -> 551), 8 of 1000 x 500 cells per = 3
+// (316 -> 281).
+void sweep_plan_throughput(const int* dims, SweepPlan* const* plans, int count);
 cudaError_t grid_setup(int N, int M);
 void launch_sweep_uz(const DevGrid& g, const DevParams& p, const SweepPlan& sp, int startidx, int endidx,
                      int solver, double* scratch, cudaStream_t s);

@@ -1252,11 +1252,18 @@ cudaError_t sweep_plan(int N, int M, SweepPlan* sp, int max_rows) {
     return cudaSuccess;
 }
 
-void sweep_plan_throughput(int N, int M, SweepPlan* sp) {
-    const int L = N > M ? N : M;
-    const int g = (L + 3 + kWL - 1) / kWL;
-    if (sp->long_grid > g) sp->long_grid = g;
-    sp->wide = 1;
+void sweep_plan_throughput(const int* dims, SweepPlan* const* plans, int count) {
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    long long total = 0;  // CTAs that give every line of every member its own warp
+    for (int k = 0; k < count; k++) total += (std::max(dims[2 * k], dims[2 * k + 1]) + 3 + kWL - 1) / kWL;
+    const long long per = std::min(std::max((total + nsm / 2) / nsm, 1LL), 4LL);
+    for (int k = 0; k < count; k++) {
+        const int g = (int)((std::max(dims[2 * k], dims[2 * k + 1]) + 3 + kWL * per - 1) / (kWL * per));
+        if (plans[k]->long_grid > g) plans[k]->long_grid = g;
+        plans[k]->wide = 1;
+    }
 }
 
 namespace {

@@ -441,7 +441,8 @@ int hyd_batch_fused_steps(hyd_batch b, long long* steps);
  * Launch shape of a handle's line sweeps: `ctas` persistent CTAs (0 or more than planned:
  * the planned number, one per SM), and with `wide` = 1 shared memory for 16 lines of up to 288
  * rows side by side in a CTA rather than of up to 96 (lines that do not fit together are swept
- * in rounds).  Batch members start at ceil((max(N, M) + 3) / 16) CTAs, wide.  Changing the shape
+ * in rounds).  Batch members start at ceil((max(N, M) + 3) / (16 k)) CTAs, wide, with k = 1 to 4
+ * by the batch's lines (all members' CTAs together about one per SM).  Changing the shape
  * drops the captured step graphs (the next step captures anew).  Results do not depend on
  * the shape.  No reference counterpart (the reference launches one block per line);
  * hydist.tune picks shapes by timing.

@@ -1107,7 +1107,7 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
         start_idx = 3;
         end_idx = s->M - 1;
     }
-    { PHASE(PH_COEF_UZ); launch_coef_bnd(g, p, 0, 3, st); }
+    { PHASE(PH_COEF_UZ); launch_coef_bnd(g, p, 0, 3, s->plan.wide, st); }
     { PHASE(PH_SWEEP_UZ); launch_sweep_uz(g, p, s->plan, start_idx, end_idx, s->solver, s->sweep_scratch, st); }
     // span-limited passes: the half-step's water budget beside the smoothing and explicit v
     // (joined before the row resets change the mask); whole-grid passes keep it in the
@@ -1126,7 +1126,7 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     const int mom = !fh && !force, msm = mom && !s->plan.wide && mom_smooths(g);
     if (msm) {
         PHASE(PH_EXPL_V);
-        launch_mom(g, p, 1, 1, s->scratch_u, st);
+        launch_mom(g, p, 1, 1, s->plan.wide, s->scratch_u, st);
         std::swap(g.t_u, s->scratch_u);
     } else {
         { PHASE(PH_SMOOTH); launch_smooth(g, p, 1, s->scratch_u, fh, 0, 0, fh, st); }
@@ -1159,18 +1159,18 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     if (overlap) {
         cudaEventRecord(s->ev_fork, st);
         cudaStreamWaitEvent(s->side, s->ev_fork, 0);
-        { PHASE_ON(PH_COEF_FSJ, s->side); launch_coef_fsj(g, p, 0, s->side); }
+        { PHASE_ON(PH_COEF_FSJ, s->side); launch_coef_fsj(g, p, 0, s->plan.wide, s->side); }
         { PHASE_ON(PH_FS_J, s->side); launch_fs_sweep_j(g, p, s->plan, 0, s->solver, s->fs_scratch, s->side); }
         { PHASE_ON(PH_UPDATE_FS, s->side); launch_update_fs(g, fsd, s->side); }
         cudaEventRecord(s->ev_join, s->side);
     } else if (sed1) {
         if (!(sed1 && fuse1)) { PHASE(PH_VTH); launch_vth_hesok(g, p, fsd, 0, st); }
-        { PHASE(PH_COEF_FSJ); launch_coef_fsj(g, p, 0, st); }
+        { PHASE(PH_COEF_FSJ); launch_coef_fsj(g, p, 0, s->plan.wide, st); }
         { PHASE(PH_FS_J); launch_fs_sweep_j(g, p, s->plan, 0, s->solver, s->fs_scratch, st); }
         { PHASE(PH_UPDATE_FS); launch_update_fs(g, fsd, st); }
     }
     // ---- half-step 2: implicit along j (rows), explicit u
-    { PHASE(PH_BOUNDARY); launch_coef_bnd(g, p, 1, overlap ? 1 : 3, st); }
+    { PHASE(PH_BOUNDARY); launch_coef_bnd(g, p, 1, overlap ? 1 : 3, s->plan.wide, st); }
     start_idx = 2;
     end_idx = s->N;
     if (p.channel && s->P.kenhhepng == 1) {
@@ -1191,7 +1191,7 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     }
     if (mom) {
         PHASE(PH_EXPL_U);
-        launch_mom(g, p, 0, msm, s->scratch_v, st);
+        launch_mom(g, p, 0, msm, s->plan.wide, s->scratch_v, st);
         if (msm) std::swap(g.t_v, s->scratch_v);
     } else {
         { PHASE(PH_COEF_EU); launch_coef_eu(g, p, st); }
@@ -2004,7 +2004,7 @@ int fused_build(HydBatch* b) {
         counts[BP_EV].push_back(N - 1);
         counts[BP_RR].push_back(N);
         counts[BP_RC].push_back(M);
-        counts[BP_PF].push_back(row_warp_ctas(g0, N + 1) + 32 + 8);
+        counts[BP_PF].push_back(row_warp_ctas(g0, N + 1) + 32 + 16);
         counts[BP_FSJC].push_back(((N - 1) * 32 + 255) / 256);
         counts[BP_UFS].push_back(row_warp_ctas(g0, N) + 2);
         lines[BL_UZ].push_back(M - 1);

@@ -113,6 +113,36 @@ __host__ __device__ __forceinline__ int row_warp_ctas(const DevGrid& g, int rows
     return (rows * g.wpr * 32 + 255) / 256;
 }
 
+// Row-lane mapping: w warps per row.  Thread -> row i0 + (warp / w), first cell offset
+// (warp % w) * 32 + lane, stride w * 32.  The extended-span kernels take g.wpr warps per row, so
+// that a row's span is covered in one pass.
+struct RowLane {
+    int i, off, stride;
+    __device__ __forceinline__ RowLane(int i0, int w, int bx) {
+        const int gw = (bx * blockDim.x + threadIdx.x) >> 5;
+        i = i0 + gw / w;
+        off = (gw % w) * 32 + (threadIdx.x & 31);
+        stride = w * 32;
+    }
+    __device__ __forceinline__ RowLane(const DevGrid& g, int i0, int bx) : RowLane(i0, g.wpr, bx) {}
+};
+
+// Launch shape of the row-major coefficient kernels (untiled): CTAs of `threads`, wpc warps per
+// row.  A row's cells in one pass and few warps per CTA while the device has SMs and warps to
+// spare: with one warp per row in CTAs of 8, the 211 rows of an island reach ran on 27 SMs,
+// three passes each (14.6 us).  From about a wave on, and for reaches that share the device, one
+// warp per row (4096 x 2048: 46 us against 50 with several; 16 reaches 262 us a step against
+// 280).
+struct CoefShape {
+    int threads, wpc;
+};
+inline CoefShape coef_shape(const DevGrid& g) {
+    constexpr int kSms = 148;
+    const int wpc = g.N * g.wpr <= 16 * kSms ? g.wpr : 1;
+    const int warps = g.N * wpc;
+    return CoefShape{warps >= 8 * kSms ? 256 : (warps >= 4 * kSms ? 128 : 64), wpc};
+}
+
 // A batch of reaches stepped by batched launches: member m's grid and parameters (device
 // arrays), and for one launch the first CTA of each member's share (bstart[m], with
 // bstart[nm] the launch's CTAs).  Every CTA of a batched launch works for one member.
@@ -362,7 +392,7 @@ void launch_widen_spans(const DevGrid& g, cudaStream_t s);
 // Span-limited steps: one component's explicit momentum (dir 1: v, dir 0: u), with `smooth` also
 // the smoothing of the other, swept component into out (else it is smoothed already).
 int mom_smooths(const DevGrid& g);
-void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, double* out, cudaStream_t s);
+void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, int shared, double* out, cudaStream_t s);
 void launch_explicit_v(const DevGrid& g, const DevParams& p, int threads, cudaStream_t s);
 void launch_explicit_u(const DevGrid& g, const DevParams& p, int threads, cudaStream_t s);
 void launch_coef_eu(const DevGrid& g, const DevParams& p, cudaStream_t s);
@@ -390,8 +420,9 @@ void launch_post_fused(const DevGrid& g, const DevParams& p, int rows, int vth, 
 // The first launch of half-step `half`: its line coefficients (UZ column-major / VZ
 // row-major) and its boundary values (`writes`: 1 velocities/levels, 2 inflow
 // concentrations, 3 both; ignored in channel mode).  Half-step 1 also advances the clock.
-void launch_coef_bnd(const DevGrid& g, const DevParams& p, int half, int writes, cudaStream_t s);
-void launch_coef_fsj(const DevGrid& g, const DevParams& p, int half, cudaStream_t s);
+// shared: the device is shared with other reaches (batch members), whose work fills it.
+void launch_coef_bnd(const DevGrid& g, const DevParams& p, int half, int writes, int shared, cudaStream_t s);
+void launch_coef_fsj(const DevGrid& g, const DevParams& p, int half, int shared, cudaStream_t s);
 void launch_fs_sweep_j(const DevGrid& g, const DevParams& p, const SweepPlan& sp, int half, int solver,
                        double* scratch, cudaStream_t s);
 void launch_fs_sweep_i(const DevGrid& g, const DevParams& p, const SweepPlan& sp, int half, int solver,

@@ -166,19 +166,32 @@ struct BndSeg {
     double value, cv;
 };
 
+// Every load that does not need another's value is issued before the first test (the tables of
+// an edge without any are null): one memory round trip instead of four in a row.
 __device__ __forceinline__ BndSeg bnd_segment(const DevGrid& g, const EdgeArgs& a, double t) {
     BndSeg s{1, 0, 0, 0.0, 0.0};
-    if (a.moc[a.location] <= 0) return s;
     const int tt = g.total_time;
     const int t1 = (int)(t / 3600);
     const double t2 = (t - (3600.0 * t1)) / 3600.0;
     const int seg_no = 0;
-    s.lo = a.dau[a.location * HYD_SEGL];
-    s.hi = a.cuoi[a.location * HYD_SEGL];
-    s.value = a.bcv[seg_no * tt + t1] * (1.0 - t2) + a.bcv[seg_no * tt + t1 + 1] * t2;
-    if (a.btype[seg_no] == 2) {
+    const int moc = a.moc[a.location], lo = a.dau[a.location * HYD_SEGL], hi = a.cuoi[a.location * HYD_SEGL],
+              type = a.btype[seg_no];
+    double b0 = 0.0, b1 = 0.0, c0 = 0.0, c1 = 0.0;
+    if (a.bcv) {
+        b0 = a.bcv[seg_no * tt + t1];
+        b1 = a.bcv[seg_no * tt + t1 + 1];
+    }
+    if (a.ccv) {
+        c0 = a.ccv[seg_no * tt + t1];
+        c1 = a.ccv[seg_no * tt + t1 + 1];
+    }
+    if (moc <= 0) return s;
+    s.lo = lo;
+    s.hi = hi;
+    s.value = b0 * (1.0 - t2) + b1 * t2;
+    if (type == 2) {
         s.kind = 1;
-        s.cv = a.ccv[seg_no * tt + t1] * (1.0 - t2) + a.ccv[seg_no * tt + t1 + 1] * t2;
+        s.cv = c0 * (1.0 - t2) + c1 * t2;
     } else {
         s.kind = 2;
     }
@@ -231,6 +244,9 @@ __device__ void bnd_apply(const DevGrid& g, const EdgeArgs& a, const BndRec& r, 
 // the up edge, which threads past the first warp repeat in the reference.  `writes`
 // selects the arrays written (the same order applies within each array), so the
 // concentration part can run after work that the velocity/level part need not wait for.
+// Only the open segment's indices are walked (an index outside it has nothing to apply); over
+// every index of the edge, 64 threads took five rounds of loads on a 1048 x 980 grid, and this
+// CTA was the longest of its launch.
 __device__ void boundary_body(const DevGrid& g, double t, int writes = kBndAll) {
     __shared__ BndRec s_rec[4][2];
     const int N = g.N, M = g.M;
@@ -240,16 +256,20 @@ __device__ void boundary_body(const DevGrid& g, double t, int writes = kBndAll) 
         const EdgeArgs a = edge_args(g, e);
         const int far = a.isU ? M : N;
         const BndSeg sg = bnd_segment(g, a, t);
+        const int lo = max(sg.lo, 2), hi = min(sg.hi, imax);
+        // the corners' records: nothing where the segment does not reach them
+        if (r == 0 && (lo > 2 || hi < 2)) s_rec[e][0] = BndRec{0, 0.0, 0.0};
+        if (r == 0 && (lo > far || hi < far)) s_rec[e][1] = BndRec{0, 0.0, 0.0};
         // four indices at a time: their loads issue before any of their stores
         constexpr int U = 4;
-        for (int i0 = 2 + r; i0 <= imax; i0 += U * Q) {
+        for (int i0 = lo + r; i0 <= hi; i0 += U * Q) {
             BndRec rec[U];
 #pragma unroll
             for (int u = 0; u < U; u++) rec[u] = bnd_at(g, a, sg, i0 + u * Q);
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const int i = i0 + u * Q;
-                if (i > imax) break;
+                if (i > hi) break;
                 if (i == 2) s_rec[e][0] = rec[u];
                 else if (i == far) s_rec[e][1] = rec[u];
                 else bnd_apply(g, a, rec[u], i, writes);
@@ -436,28 +456,24 @@ __device__ __forceinline__ void vz_cell_coeffs(const DevGrid& g, const DevParams
 // small grids' launches, whose stencil loads it serves.
 // bx, gx: the CTA's index among the launch's CTAs of this grid and their count (blockIdx.x
 // and gridDim.x of a launch for one grid; a member's share of a batched launch).
+// wpc: warps per row of the untiled form.
 template <int KIND, int TILE, class R>
-__device__ __forceinline__ void coef_bnd_body(const DevGrid& g, const DevParams& p, int writes, int bx, int gx) {
+__device__ __forceinline__ void coef_bnd_body(const DevGrid& g, const DevParams& p, int writes, int wpc, int bx) {
     // CTA 0 takes the clock and the boundary (a chain of dependent loads, started first
     // so that it runs beside the coefficient CTAs instead of after them); the others the
     // coefficients
     if (bx == 0) {
-        __shared__ double s_t;
-        if (threadIdx.x == 0) {
-            if (KIND == 0) {  // k_clock
-                const double t1 = g.clock[2] + p.dT * 0.5;
-                const double t2 = t1 + p.dT * 0.5;
-                g.clock[0] = t1;
-                g.clock[1] = t2;
-                g.clock[2] = t2;
-                s_t = t1;
-            } else {
-                s_t = g.clock[1];
-            }
+        // every thread reads the clock; thread 0 advances it once all have (both bodies pass a
+        // CTA barrier)
+        const double t1 = KIND == 0 ? g.clock[2] + p.dT * 0.5 : g.clock[1];
+        if (p.channel) boundary_channel_body(g, p, t1);
+        else boundary_body(g, t1, writes);
+        if (KIND == 0 && threadIdx.x == 0) {  // k_clock
+            const double t2 = t1 + p.dT * 0.5;
+            g.clock[0] = t1;
+            g.clock[1] = t2;
+            g.clock[2] = t2;
         }
-        __syncthreads();
-        if (p.channel) boundary_channel_body(g, p, s_t);
-        else boundary_body(g, s_t, writes);
         return;
     }
     bx -= 1;
@@ -475,12 +491,12 @@ __device__ __forceinline__ void coef_bnd_body(const DevGrid& g, const DevParams&
             dst);
         return;
     }
-    // rows 2..N, one warp per row (several warps per row measured slower on config 4:
-    // 46 -> 50 us), lanes striding over the row's cells
-    const int i = 2 + ((bx * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    // rows 2..N, wpc warps per row (coef_shape), lanes striding over the row's cells
+    const RowLane rl(2, wpc, bx);
+    const int i = rl.i;
     if (i > g.N) return;
     const int lo = max(g.rlo[i], 2), hi = min(g.rhi[i], g.M);
-    for (int j = lo + lane; j <= hi; j += 32) {
+    for (int j = lo + rl.off; j <= hi; j += rl.stride) {
         const int pos = i * g.P + j;
         if (g.khouot[pos] != 0) continue;
         R a2, c2, d2, f1, f2, f3, f5;
@@ -508,13 +524,13 @@ __device__ __forceinline__ void coef_bnd_body(const DevGrid& g, const DevParams&
 }
 
 template <int KIND, int TILE, class R>
-__global__ void __launch_bounds__(256) k_coef_bnd(DevGrid g, DevParams p, int writes) {
-    coef_bnd_body<KIND, TILE, R>(g, p, writes, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(256) k_coef_bnd(DevGrid g, DevParams p, int writes, int wpc) {
+    coef_bnd_body<KIND, TILE, R>(g, p, writes, wpc, blockIdx.x);
 }
 template <int KIND, int TILE, class R>
 __global__ void __launch_bounds__(256) k_coef_bnd_b(BatchRef br, int writes) {
     const BatchMember bm(br);
-    coef_bnd_body<KIND, TILE, R>(bm.g, bm.p, writes, bm.bx, bm.gx);
+    coef_bnd_body<KIND, TILE, R>(bm.g, bm.p, writes, 1, bm.bx);
 }
 
 // ------------------------------------------------------------------- smoothing
@@ -584,19 +600,6 @@ __device__ __forceinline__ void reset_byte_cell(const DevGrid& g, const DevParam
     }
     g.colB[(size_t)j * g.LT + i] = (unsigned char)b;
 }
-
-// Row-lane mapping of the extended-span kernels: g.wpr warps per row, so that a row's
-// span is covered in one pass.  Thread -> row i0 + (warp / wpr), first cell offset
-// (warp % wpr) * 32 + lane, stride wpr * 32.
-struct RowLane {
-    int i, off, stride;
-    __device__ __forceinline__ RowLane(const DevGrid& g, int i0, int bx) {
-        const int gw = (bx * blockDim.x + threadIdx.x) >> 5;
-        i = i0 + gw / g.wpr;
-        off = (gw % g.wpr) * 32 + (threadIdx.x & 31);
-        stride = g.wpr * 32;
-    }
-};
 
 // The open-edge part of the water budget for one half-step, by kEdgeCtas CTAs for edge e
 // (0 up: faces j = M, 1 down: faces j = 1, 2 left: faces i = 1, 3 right: faces i = N), run
@@ -1955,7 +1958,7 @@ __device__ __forceinline__ void post_vth_cell(const DevGrid& g, const DevParams&
 // direction (nbs CTAs); and the edge concentration interpolation (kEdgeParts CTAs,
 // reading t_u / t_v where the reference reads u / v after the update).  None of the
 // three writes what another reads.
-constexpr int kEdgeParts = 8;
+constexpr int kEdgeParts = 16;
 template <int ROWS, int VTH, class R>
 __device__ __forceinline__ void post_fused_body(const DevGrid& g, const DevParams& p, int nbp, int nbs, int bx,
                                                 int gx) {
@@ -2522,24 +2525,27 @@ void launch_init_kernels(const DevGrid& g, const DevParams& p, const int* keep_m
 }
 
 
-void launch_coef_bnd(const DevGrid& g, const DevParams& p, int half, int writes, cudaStream_t s) {
-    // the tiled form: kTileRows rows per CTA; the row form: one warp per row (the same count)
-    const int nb = ((g.N - 1) * 32 + 255) / 256 + 1;
-    const int nbr = nb;
-    if (p.mixed) {
-        if (half == 1) k_coef_bnd<1, 0, float><<<nbr, 256, 0, s>>>(g, p, writes);
-        else if (g.tile_cols) k_coef_bnd<0, 1, float><<<nb, 256, 0, s>>>(g, p, writes);
-        else k_coef_bnd<0, 0, float><<<nbr, 256, 0, s>>>(g, p, writes);
-    } else {
-        if (half == 1) k_coef_bnd<1, 0, double><<<nbr, 256, 0, s>>>(g, p, writes);
-        else if (g.tile_cols) k_coef_bnd<0, 1, double><<<nb, 256, 0, s>>>(g, p, writes);
-        else k_coef_bnd<0, 0, double><<<nbr, 256, 0, s>>>(g, p, writes);
-    }
+void launch_coef_bnd(const DevGrid& g, const DevParams& p, int half, int writes, int shared, cudaStream_t s) {
+    // the tiled form: kTileRows rows per CTA of 256; the row form by coef_shape
+    const bool tile = half == 0 && g.tile_cols;
+    const CoefShape c = tile || shared ? CoefShape{256, 1} : coef_shape(g);
+    const int nb = ((g.N - 1) * c.wpc * 32 + c.threads - 1) / c.threads + 1;
+    void (*const k[2][3])(DevGrid, DevParams, int, int) = {
+        {k_coef_bnd<0, 0, double>, k_coef_bnd<0, 1, double>, k_coef_bnd<1, 0, double>},
+        {k_coef_bnd<0, 0, float>, k_coef_bnd<0, 1, float>, k_coef_bnd<1, 0, float>}};
+    k[p.mixed ? 1 : 0][half == 1 ? 2 : (tile ? 1 : 0)]<<<nb, c.threads, 0, s>>>(g, p, writes, c.wpc);
     hyd_kernel_launches_add(1);
 }
 
 // Elementwise kernels: the whole grid (`full`), or one warp per row over its extended span.
 static int row_warps_blocks(const DevGrid& g, int rows) { return row_warp_ctas(g, rows); }
+// Threads of a span kernel's CTA for `rows` rows: 256, or fewer while that leaves SMs without a
+// CTA (a 211 x 157 reach is 107 CTAs of 256: the explicit momentum took 12.2 us on 107 SMs).
+static int row_threads(const DevGrid& g, int rows) {
+    const int nb = row_warp_ctas(g, rows);
+    return nb >= 2 * scan_grid() ? 256 : (nb >= scan_grid() ? 128 : 64);
+}
+static int row_ctas(const DevGrid& g, int rows, int threads) { return (rows * g.wpr * 32 + threads - 1) / threads; }
 
 void launch_smooth(const DevGrid& g, const DevParams& p, int isU, double* out, int full, int bytes, int fs_bnd,
                    int budget, cudaStream_t s) {
@@ -2601,11 +2607,12 @@ void launch_explicit_u(const DevGrid& g, const DevParams& p, int threads, cudaSt
 // the device (the callers leave it apart there: 16 reaches 297 us joined, 284 apart).
 int mom_smooths(const DevGrid& g) { return row_warps_blocks(g, g.N + 3) <= 4 * scan_grid(); }
 
-void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, double* out, cudaStream_t s) {
+void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, int shared, double* out, cudaStream_t s) {
     void (*const k[2][2][2])(DevGrid, DevParams, double*) = {
         {{k_mom_span<0, 0, double>, k_mom_span<0, 0, float>}, {k_mom_span<0, 1, double>, k_mom_span<0, 1, float>}},
         {{k_mom_span<1, 0, double>, k_mom_span<1, 0, float>}, {k_mom_span<1, 1, double>, k_mom_span<1, 1, float>}}};
-    k[dir ? 1 : 0][smooth ? 1 : 0][p.mixed ? 1 : 0]<<<row_warps_blocks(g, g.N + 3), 256, 0, s>>>(g, p, out);
+    const int t = shared ? 256 : row_threads(g, g.N + 3);
+    k[dir ? 1 : 0][smooth ? 1 : 0][p.mixed ? 1 : 0]<<<row_ctas(g, g.N + 3, t), t, 0, s>>>(g, p, out);
     hyd_kernel_launches_add(1);
 }
 

@@ -873,17 +873,18 @@ __device__ __forceinline__ void fsi_cell_coeffs(const DevGrid& g, const DevParam
     dd = R(FSd) / (R(p.dT) * R(0.5)) - qq + pp + src;
 }
 
-// FSj rows of every interior wet cell (columns 3..M-1), one warp per row of the grid over
-// the row's span, written column-major (colT arrays 0..3 in R: aa bb cc dd), with TILE
+// FSj rows of every interior wet cell (columns 3..M-1), wpc warps per row of the grid over
+// the row's span (coef_shape), written column-major (colT arrays 0..3 in R: aa bb cc dd), with TILE
 // through a tile.
 template <int TILE, class R>
-__device__ __forceinline__ void coef_fsj_body(const DevGrid& g, const DevParams& p, int half, int bx) {
+__device__ __forceinline__ void coef_fsj_body(const DevGrid& g, const DevParams& p, int half, int wpc, int bx) {
     const double t = g.clock[half];
     if constexpr (!TILE) {
-        const int i = 2 + ((bx * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+        const RowLane rl(2, wpc, bx);
+        const int i = rl.i;
         if (i > g.N) return;
         const int lo = max(g.rlo[i], 3), hi = min(g.rhi[i], g.M - 1);
-        for (int j = lo + lane; j <= hi; j += 32) {
+        for (int j = lo + rl.off; j <= hi; j += rl.stride) {
             const int pos = i * g.P + j;
             if (g.khouot[pos] != 0) continue;
             R aa, bb, cc, dd;
@@ -909,13 +910,13 @@ __device__ __forceinline__ void coef_fsj_body(const DevGrid& g, const DevParams&
 }
 
 template <int TILE, class R>
-__global__ void __launch_bounds__(256) k_coef_fsj(DevGrid g, DevParams p, int half) {
-    coef_fsj_body<TILE, R>(g, p, half, blockIdx.x);
+__global__ void __launch_bounds__(256) k_coef_fsj(DevGrid g, DevParams p, int half, int wpc) {
+    coef_fsj_body<TILE, R>(g, p, half, wpc, blockIdx.x);
 }
 template <int TILE, class R>
 __global__ void __launch_bounds__(256) k_coef_fsj_b(BatchRef br, int half) {
     const BatchMember bm(br);
-    coef_fsj_body<TILE, R>(bm.g, bm.p, half, bm.bx);
+    coef_fsj_body<TILE, R>(bm.g, bm.p, half, 1, bm.bx);
 }
 
 // Segments of a sediment line and their row offsets (one row per interior cell
@@ -1299,15 +1300,12 @@ void fs_sweep(int dir, const DevGrid& g, const DevParams& p, const SweepPlan& sp
 }
 }  // namespace
 
-void launch_coef_fsj(const DevGrid& g, const DevParams& p, int half, cudaStream_t s) {
-    const int nb = ((g.N - 1) * 32 + 255) / 256;
-    if (p.mixed) {
-        if (g.tile_cols) k_coef_fsj<1, float><<<nb, 256, 0, s>>>(g, p, half);
-        else k_coef_fsj<0, float><<<nb, 256, 0, s>>>(g, p, half);
-    } else {
-        if (g.tile_cols) k_coef_fsj<1, double><<<nb, 256, 0, s>>>(g, p, half);
-        else k_coef_fsj<0, double><<<nb, 256, 0, s>>>(g, p, half);
-    }
+void launch_coef_fsj(const DevGrid& g, const DevParams& p, int half, int shared, cudaStream_t s) {
+    const CoefShape c = g.tile_cols || shared ? CoefShape{256, 1} : coef_shape(g);
+    const int nb = ((g.N - 1) * c.wpc * 32 + c.threads - 1) / c.threads;
+    void (*const k[2][2])(DevGrid, DevParams, int, int) = {{k_coef_fsj<0, double>, k_coef_fsj<1, double>},
+                                                           {k_coef_fsj<0, float>, k_coef_fsj<1, float>}};
+    k[p.mixed ? 1 : 0][g.tile_cols ? 1 : 0]<<<nb, c.threads, 0, s>>>(g, p, half, c.wpc);
     hyd_kernel_launches_add(1);
 }
 

@@ -1201,7 +1201,7 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     { PHASE(PH_SMOOTH); launch_smooth(g, p, 1, s->scratch_u, fh, 1, overlap, 0, st); }
     std::swap(g.t_u, s->scratch_u);
     if (!fh) cudaStreamWaitEvent(st, s->ev_bjoin, 0);
-    { PHASE(PH_RESET_COLS); launch_reset_cols(g, p, 0, s->thr_c, st); }
+    { PHASE(PH_RESET_COLS); launch_reset_cols(g, p, 0, st); }
     if (!fh) {
         PHASE(PH_POST);
         launch_post_fused(g, p, 1, sed2 && fuse1, st);
@@ -1847,7 +1847,8 @@ struct BatchFused {
     int grid = 0;
     double* gscr = nullptr;     // sweep rows of lines too long for shared memory (if any)
     double* gscr_fs = nullptr;  // the same for the sediment sweep beside the main chain
-    int thr_r = 64, thr_c = 64;
+    int thr_r = 64;
+    int rcw = 1;  // columns per CTA of the column resets
     size_t sm_ev = 0, sm_rr = 0, sm_rc = 0, sm_pf = 0;
     cudaStream_t st = nullptr, side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
@@ -1979,7 +1980,13 @@ int fused_build(HydBatch* b) {
     std::vector<double*> outs[4];
     std::vector<int> counts[BP_COUNT];
     std::vector<int> lines[BL_COUNT], firsts[BL_COUNT];
-    int Nmax = 0, Mmax = 0;
+    int Nmax = 0, Mmax = 0, cols = 0;
+    for (HydSim* s : b->members) {
+        Nmax = std::max(Nmax, s->N);
+        Mmax = std::max(Mmax, s->M);
+        cols += s->M;
+    }
+    f.rcw = reset_col_warps(Nmax, cols);
     for (HydSim* s : b->members) {
         const DevGrid g0 = s->g;
         double *A = g0.t_u, *Bu = s->scratch_u, *C = g0.t_v, *D = s->scratch_v;
@@ -2003,7 +2010,7 @@ int fused_build(HydBatch* b) {
         counts[BP_SM_FSB].push_back(rw + 1);
         counts[BP_EV].push_back(N - 1);
         counts[BP_RR].push_back(N);
-        counts[BP_RC].push_back(M);
+        counts[BP_RC].push_back((M + f.rcw - 1) / f.rcw);
         counts[BP_PF].push_back(row_warp_ctas(g0, N + 1) + 32 + 16);
         counts[BP_FSJC].push_back(((N - 1) * 32 + 255) / 256);
         counts[BP_UFS].push_back(row_warp_ctas(g0, N) + 2);
@@ -2015,15 +2022,12 @@ int fused_build(HydBatch* b) {
         firsts[BL_FSJ].push_back(3);
         lines[BL_FSI].push_back(N - 3);
         firsts[BL_FSI].push_back(3);
-        Nmax = std::max(Nmax, N);
-        Mmax = std::max(Mmax, M);
         f.thr_r = std::max(f.thr_r, s->thr_r);
-        f.thr_c = std::max(f.thr_c, s->thr_c);
         size_t ev, rr, rc, pf;
         line_smem(N, M, &ev, &rr, &rc, &pf);
         f.sm_ev = std::max(f.sm_ev, ev);
         f.sm_rr = std::max(f.sm_rr, rr);
-        f.sm_rc = std::max(f.sm_rc, rc);
+        f.sm_rc = std::max(f.sm_rc, f.rcw * rc);
         f.sm_pf = std::max(f.sm_pf, pf);
     }
     // one device block: grids, parameters, output pointers, CTA starts, line lists
@@ -2128,7 +2132,7 @@ void fused_launch_step(HydBatch* b, int sed1, int sed2, int bed) {
     if (sed1) cudaStreamWaitEvent(st, f.join, 0);
     launch_smooth_batch(BR(1, sed1 ? BP_SM_FSB : BP_SM), f.ctas[sed1 ? BP_SM_FSB : BP_SM], 1, f.outs[3], 1, sed1, 0,
                         st);
-    launch_reset_batch(BR(0, BP_RC), f.ctas[BP_RC], 0, f.thr_c, f.sm_rc, st);
+    launch_reset_batch(BR(0, BP_RC), f.ctas[BP_RC], 0, 32 * f.rcw, f.sm_rc, st);
     launch_post_fused_batch(BR(0, BP_PF), f.ctas[BP_PF], 1, sed2, mx, f.sm_pf, st);
     if (sed2) {
         launch_fs_sweep_batch(1, BL(0, BL_FSI), f.plan, 1, f.solver, mx, f.gscr, f.grid, st);

@@ -583,7 +583,7 @@ __device__ __forceinline__ void smooth_cell(const DevGrid& g, const DevParams& p
     out[gp] = smooth_value(g, p, isU, i, j);
 }
 
-// The column-major reset byte of cell (i, j) for the column resets that follow (k_reset
+// The column-major reset byte of cell (i, j) for the column resets that follow (k_reset_cols
 // columns): mask | (t_z > z, rows 2..N) << 2 | (wet with H <= H_TINH, rows 2..N) << 3,
 // after update_h_moi (support_funcs.cu:60-73) on the wet cells of 1..N x 1..M.
 __device__ __forceinline__ void reset_byte_cell(const DevGrid& g, const DevParams& p, int i, int j) {
@@ -1299,16 +1299,65 @@ __device__ __forceinline__ void pack_wet_ints(const int* row, int a, int b, unsi
     }
 }
 
+// Bits t with a <= c + t <= b.
+__device__ __forceinline__ unsigned range_bits(int c, int a, int b) {
+    if (c > b || c + 31 < a) return 0u;
+    unsigned m = 0xffffffffu;
+    if (c < a) m &= 0xffffffffu << (a - c);
+    if (c + 31 > b) m &= 0xffffffffu >> (c + 31 - b);
+    return m;
+}
+
+// The maximal runs of set bits within cells a..b of nq packed words (bit t of word q is cell
+// org + 32 q + t), in order, into dau / cuoi / moc, by one warp; runs that start at L-1 or L
+// are left out.  Each lane takes a word: the runs before its own come from a prefix sum of the
+// lanes' start and end counts (one lane walking the words of a 1048-cell line was 34 rounds).
+__device__ __forceinline__ void warp_runs(const DevGrid& g, const unsigned* words, int nq, int org, int a, int b, int L,
+                                          int* dau, int* cuoi, int* moc) {
+    const int lane = threadIdx.x & 31;
+    int runs = 0, closed = 0;
+    for (int q0 = 0; q0 < nq; q0 += 32) {
+        const int q = q0 + lane, c = org + 32 * q;
+        unsigned cur = 0, prev = 0, next = 0;
+        if (q < nq) {
+            cur = words[q] & range_bits(c, a, b);
+            if (q > 0) prev = words[q - 1] & range_bits(c - 32, a, b);
+            if (q + 1 < nq) next = words[q + 1] & range_bits(c + 32, a, b);
+        }
+        unsigned starts = cur & ~((cur << 1) | (prev >> 31)) & range_bits(c, a, L - 2);
+        unsigned ends = cur & ~((cur >> 1) | (next << 31));
+        const int own = __popc(starts) | (__popc(ends) << 16);
+        int inc = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += v;
+        }
+        const int upto = runs + (inc & 0xffff);  // runs started up to this word
+        int r = upto - __popc(starts);
+        for (; starts; starts &= starts - 1, r++) {
+            if (r < HYD_SEGL) dau[r] = c + __ffs(starts) - 1;
+            else flag_status(g, HYD_ST_SEG_OVERFLOW);
+        }
+        r = closed + ((inc - own) >> 16);
+        for (; ends; ends &= ends - 1, r++)
+            if (r < upto && r < HYD_SEGL) cuoi[r] = c + __ffs(ends) - 1;
+        const int tot = __shfl_sync(0xffffffffu, inc, 31);
+        runs += tot & 0xffff;
+        closed += tot >> 16;
+    }
+    if (lane == 0) *moc = runs < HYD_SEGL ? runs : HYD_SEGL;
+}
+
 // Wet-segment scan of one line by one warp (Find_Calculation_limits_Horizontal/Vertical,
 // support_funcs.cu:230-335).  The serial while-loop there yields the maximal runs of
 // khouot == 0 within [2, L] in order, except runs starting at L-1 or L, which it skips.
 // Cells a..b are tested with wet(k); every other cell is dry.  The warp packs the wet
 // flags into 32-cell words (words: (b - a) / 32 + 2 entries of shared memory; mask bytes
-// and mask rows with wide loads), then lane 0 walks the run starts and ends word by word.
+// and mask rows with wide loads) and takes their runs.
 template <class Wet>
 __device__ void warp_scan_line(const DevGrid& g, Wet wet, int a, int b, int L, unsigned* words, int* dau, int* cuoi,
                                int* moc) {
-    const int lane = threadIdx.x & 31;
     if (a < 2) a = 2;
     if (b > L) b = L;
     int origin = 2;
@@ -1326,49 +1375,9 @@ __device__ void warp_scan_line(const DevGrid& g, Wet wet, int a, int b, int L, u
         }
     }
     __syncwarp();
-    if (lane == 0) {
-        int nseg = 0;
-        int open_start = -1;
-        for (int w = w0; b >= a && w <= w1; w++) {
-            const unsigned cur = words[w - w0];
-            const unsigned prev = w > w0 ? words[w - w0 - 1] : 0u;
-            const unsigned next = w < w1 ? words[w - w0 + 1] : 0u;
-            unsigned starts = cur & ~((cur << 1) | (prev >> 31));
-            unsigned ends = cur & ~((cur >> 1) | (next << 31));
-            const int c0 = origin + 32 * w;
-            // events in position order; a run's start precedes or equals its end
-            while (starts | ends) {
-                if (open_start < 0) {
-                    if (!starts) break;
-                    open_start = c0 + __ffs(starts) - 1;
-                    starts &= starts - 1;
-                } else {
-                    if (!ends) break;  // the run continues into the next word
-                    const int e = c0 + __ffs(ends) - 1;
-                    ends &= ends - 1;
-                    if (open_start <= L - 2) {
-                        if (nseg < HYD_SEGL) {
-                            dau[nseg] = open_start;
-                            cuoi[nseg] = e;
-                        } else {
-                            flag_status(g, HYD_ST_SEG_OVERFLOW);
-                        }
-                        nseg++;
-                    }
-                    open_start = -1;
-                }
-            }
-        }
-        *moc = nseg < HYD_SEGL ? nseg : HYD_SEGL;
-    }
+    warp_runs(g, words, b >= a ? w1 - w0 + 1 : 0, origin + 32 * w0, a, b, L, dau, cuoi, moc);
     __syncwarp();
 }
-
-struct WetShared {  // staged mask: cell k at kh[k - k0]
-    const signed char* kh;
-    int k0;
-    __device__ bool operator()(int k) const { return kh[k - k0] == 0; }
-};
 
 struct WetGlobal {  // mask in HBM: cell k at kh[base + k * along]
     const int* kh;
@@ -1385,197 +1394,305 @@ struct WetBytes {
     const unsigned char* col;
 };
 
-// Words of each k_reset bitset: one bit per cell of a line.
+// Words of each reset bitset: one bit per cell of a line.
 __host__ __device__ __forceinline__ int reset_words(int L) { return (L + 3) / 32 + 2; }
+constexpr int kResetSets = 5;
 
 // update_h_moi (support_funcs.cu:60-73) and Reset_states_horizontal/_vertical
 // (support_funcs.cu:75-186) for one line.  ROWS: line = row i (1..N), cells j (2..M);
 // otherwise line = column j (1..M), cells i (2..N).
 // Cells whose mask is 2 never change (only 0 <-> 1 transitions exist), so each line is
 // staged in shared memory over its span [lo, hi] of cells that are not 2, widened by one
-// cell: nothing outside can act or be acted on.
+// cell: nothing outside can act or be acted on.  A line is five bitsets (bit t of word q is
+// cell org + 32 q + t): t_z > z, mask 1, mask 0, wet with H <= H_TINH, and opened here.
 // The opening pass is a serial scan in the reference.  Iteration k acts when t_z[k] >
 // z[k] and a neighbour's mask is 1; the only value it passes on is through the cell k+1
 // it opens, whose t_z it sets, so iteration k+1 then tests that value (a cascade through
 // a run of 1s).  Every other iteration sees the t_z, z and mask 1s of the start of the
-// pass.  So the CTA tests t_z[k] > z[k] and the mask-1 neighbours for all cells at once
-// (bitsets), and one thread runs only the cells that pass, in increasing order, each
-// with its cascade.  The closing pass closes the cells that are wet after the opening
-// pass with H <= H_TINH: the cells wet from the start (their H is update_h_moi's) and
-// the cells just opened (H stored with the opening), known as a bitset too.
-// Rows stage the mask, t_z and z of the row (coalesced) and apply update_h_moi here.
-// Columns read the column-major byte the preceding smoothing pass wrote per cell (mask,
-// t_z > z, wet with H <= H_TINH; it also applied update_h_moi), so a column is one
-// coalesced byte read instead of strided loads.
+// pass.  So one warp finds the cells that can act from the bitsets, its lanes load the values
+// of a word's such cells together, and it runs them in increasing order, each with its cascade:
+// a cell that acts is then a few shuffles, not four dependent loads and atomics (the lines of
+// the other direction are marked after the pass, by cell).  The closing pass closes the cells
+// that are wet after the opening pass with H <= H_TINH: the cells wet from the start (their H
+// is update_h_moi's) and the cells just opened (H stored with the opening).
 // A line only changes its own cells, so its segments are rescanned here when a cell
 // changed (or when `force`); every changed cell marks its line of the other direction
 // for the rescan that follows.
-// blockDim.x is a multiple of 32: each warp pass covers whole 32-cell words.
 template <int ROWS>
-__device__ __forceinline__ void reset_body(const DevGrid& g, const DevParams& p, int force, int bx) {
-    extern __shared__ unsigned char rsm[];
-    __shared__ int s_changed;
-    const int line = 1 + bx;
-    const int P = g.P;
-    const int L = ROWS ? g.M : g.N;  // last cell index of the line
-    const int along = ROWS ? 1 : P;
-    const int base = ROWS ? line * P : line;
-    const int lo = ROWS ? g.rlo[line] : g.clo[line];
-    const int hi = ROWS ? g.rhi[line] : g.chi[line];
-    int* dau = ROWS ? g.daui + line * HYD_SEGL : g.dauj + line * HYD_SEGL;
-    int* cuoi = ROWS ? g.cuoii + line * HYD_SEGL : g.cuoij + line * HYD_SEGL;
-    int* moc = ROWS ? g.moci + line : g.mocj + line;
-    if (hi < lo) {  // no cell of the line can ever be wet
-        if (force && line >= 2 && threadIdx.x == 0) *moc = 0;
-        return;
+struct ResetLine {
+    int line, L, along, base, lo, hi, k0, k1, org, nq;
+    unsigned *c0, *one, *wet, *cl, *op;
+    __device__ __forceinline__ ResetLine(const DevGrid& g, int line_, unsigned* words) : line(line_) {
+        L = ROWS ? g.M : g.N;  // last cell index of the line
+        along = ROWS ? 1 : g.P;
+        base = ROWS ? line * g.P : line;
+        lo = ROWS ? g.rlo[line] : g.clo[line];
+        hi = ROWS ? g.rhi[line] : g.chi[line];
+        k0 = lo - 1 > 0 ? lo - 1 : 0;
+        k1 = hi + 1 < L + 2 ? hi + 1 : L + 2;
+        org = k0 & ~31;
+        nq = (k1 - org) / 32 + 1;
+        const int n = reset_words(L);
+        c0 = words;
+        one = c0 + n;
+        wet = one + n;
+        cl = wet + n;
+        op = cl + n;
     }
-    int* oflags = ROWS ? g.dirty_c : g.dirty_r;
-    int* olist = ROWS ? g.dlist_c : g.dlist_r;
-    unsigned* octr = g.dctr + (ROWS ? 1 : 0);
-    const int k0 = lo - 1 > 0 ? lo - 1 : 0;
-    const int k1 = hi + 1 < L + 2 ? hi + 1 : L + 2;
-    const int nwords = reset_words(L);
-    signed char* khs = (signed char*)rsm;                       // khs[k - k0], k in [k0, k1]
-    unsigned* c0w = (unsigned*)(rsm + ((L + 3 + 15) & ~15));    // t_z > z bits, then scan words
-    unsigned* evw = c0w + nwords;                               // cells the opening pass runs
-    unsigned* clw = evw + nwords;                               // cells the closing pass closes
-    auto khv = [&](int k) -> int { return (k >= k0 && k <= k1) ? khs[k - k0] : 2; };
-    double *H = g.H_moi, *t_z = g.t_z, *FS = g.FS;
-    const double* z = g.z;
-    int* kh = g.khouot;
-    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_changed = 0;
-    // staging: the mask and the bits of every cell of [k0, k1]
-    for (int kb0 = k0; kb0 <= k1; kb0 += T) {  // uniform over the CTA
-        const int k = kb0 + tid;
-        const bool in = k <= k1;
-        bool c0 = false, cl = false;
-        if constexpr (ROWS) {
-            if (in) {
-                const int gp = base + k;
-                const int kv = kh[gp];
-                khs[k - k0] = (signed char)kv;
-                const double tz = t_z[gp];
-                c0 = k >= 2 && k <= L && tz > z[gp];
-                if (k >= 1 && k <= L && kv == 0) {
-                    const double hv = g.htaiz[gp] + tz;
-                    H[gp] = hv;
-                    cl = k >= 2 && hv <= p.H_TINH;
-                }
-            }
-        } else {
-            const unsigned b = in ? g.colB[(size_t)line * g.LT + k] : 2u;
-            if (in) khs[k - k0] = (signed char)(b & 3u);
-            c0 = (b >> 2) & 1u;
-            cl = (b >> 3) & 1u;
-        }
-        const unsigned c0b = __ballot_sync(0xffffffffu, c0), clb = __ballot_sync(0xffffffffu, cl);
-        const int q = (kb0 - k0 + warp * 32) >> 5;
-        if (lane == 0 && kb0 + warp * 32 <= k1) {
-            c0w[q] = c0b;
-            clw[q] = clb;
-        }
-    }
-    __syncthreads();
-    // the cells the opening pass runs: t_z > z with a neighbour whose mask is 1
-    const int nq = (k1 - k0) / 32 + 1;
-    int anyev = 0;
-    for (int q = warp; q < nq; q += T >> 5) {
-        const int k = k0 + q * 32 + lane;
-        const bool ev = ((c0w[q] >> lane) & 1u) && (khv(k - 1) == 1 || khv(k + 1) == 1);
-        const unsigned bits = __ballot_sync(0xffffffffu, ev);
-        if (lane == 0) evw[q] = bits;
-        anyev |= bits != 0;
-    }
-    // opening pass (loop 1), serial over those cells
+    // no cell of the line can ever be wet
+    __device__ __forceinline__ bool empty() const { return hi < lo; }
+    __device__ __forceinline__ int* moc(const DevGrid& g) const { return ROWS ? g.moci + line : g.mocj + line; }
     // interior cells opened / closed here change the domain's water volume (the budget)
-    const bool interior_line = line >= 2 && line <= (ROWS ? g.N : g.M);
-    double opened = 0.0;
-    if (__syncthreads_or(anyev) && warp == 0) {
+    __device__ __forceinline__ bool interior(const DevGrid& g) const { return line >= 2 && line <= (ROWS ? g.N : g.M); }
+    __device__ __forceinline__ bool is_one(int k) const {
+        const int t = k - org;
+        return t >= 0 && t < 32 * nq && ((one[t >> 5] >> (t & 31)) & 1u);
+    }
+    __device__ __forceinline__ size_t byte_of(const DevGrid& g, int k) const {
+        return ROWS ? (size_t)k * g.LT + line : (size_t)line * g.LT + k;
+    }
+
+    // The opening pass, by one warp.
+    __device__ __forceinline__ void open_pass(const DevGrid& g, const DevParams& p) const {
+        const int lane = threadIdx.x & 31;
+        double *H = g.H_moi, *t_z = g.t_z, *FS = g.FS;
+        const double *z = g.z, *ht = g.htaiz;
         const int kb = k1 < L ? k1 : L;
         int done = -1;
-        auto open = [&](int kk, double tzv, double fsv) {
+        double opened = 0.0;
+        auto open = [&](int kk, double tzv, double fsv, double hz) {
             const int gq = base + kk * along;
-            const double hv = g.htaiz[gq] + tzv;
+            const double hv = hz + tzv;
             t_z[gq] = tzv;
             H[gq] = hv;
-            kh[gq] = 0;
-            g.colB[ROWS ? (size_t)kk * g.LT + line : (size_t)line * g.LT + kk] = 0;  // mask bits of the byte
-            khs[kk - k0] = 0;
+            g.khouot[gq] = 0;
+            g.colB[byte_of(g, kk)] = 0;  // mask bits of the byte
             FS[gq] = fsv;
-            if (kk >= 2 && kk <= L && hv <= p.H_TINH) clw[(kk - k0) >> 5] |= 1u << ((kk - k0) & 31);
-            if (interior_line && kk >= 2 && kk <= L) opened += hv;
-            s_changed = 1;
-            mark_dirty(oflags, olist, octr, kk);
+            const int q = (kk - org) >> 5;
+            const unsigned bit = 1u << ((kk - org) & 31);
+            one[q] &= ~bit;
+            wet[q] |= bit;
+            op[q] |= bit;
+            if (kk >= 2 && kk <= L && hv <= p.H_TINH) cl[q] |= bit;
+            if (interior(g) && kk >= 2 && kk <= L) opened += hv;
         };
         for (int q0 = 0; q0 < nq; q0 += 32) {
-            const unsigned wl = q0 + lane < nq ? evw[q0 + lane] : 0u;
-            unsigned nz = __ballot_sync(0xffffffffu, wl != 0);
-            if (lane == 0) {
-                while (nz) {
-                    const int q = q0 + __ffs(nz) - 1;
-                    nz &= nz - 1;
-                    unsigned w = evw[q];
-                    while (w) {
-                        int m = k0 + q * 32 + __ffs(w) - 1;
-                        w &= w - 1;
-                        if (m <= done) continue;  // already run inside a cascade
-                        const double tzv = t_z[base + m * along], fsv = FS[base + m * along];
-                        bool act = true;
-                        for (;;) {
-                            done = m;
-                            if (!act) break;
-                            bool right = false;
-                            if (khv(m - 1) == 1) open(m - 1, tzv, fsv);
-                            if (khv(m + 1) == 1) {
-                                open(m + 1, tzv, fsv);
-                                right = true;
-                            }
-                            if (!right || m + 1 > kb) break;
-                            m++;  // the opened cell now holds tzv
-                            act = tzv > z[base + m * along];
+            const int q = q0 + lane;
+            unsigned ev = 0;
+            if (q < nq) {
+                const unsigned o = one[q], ol = q > 0 ? one[q - 1] : 0u, orr = q + 1 < nq ? one[q + 1] : 0u;
+                ev = c0[q] & ((o << 1) | (ol >> 31) | (o >> 1) | (orr << 31));
+            }
+            for (unsigned nz = __ballot_sync(0xffffffffu, ev != 0); nz; nz &= nz - 1) {
+                const int wl = __ffs(nz) - 1;
+                const int c = org + 32 * (q0 + wl);
+                unsigned w = __shfl_sync(0xffffffffu, ev, wl);
+                double tz = 0.0, fs = 0.0, zr = 0.0, hl = 0.0, hr = 0.0;
+                if ((w >> lane) & 1u) {
+                    const int gm = base + (c + lane) * along;
+                    tz = t_z[gm];
+                    fs = FS[gm];
+                    zr = z[gm + along];
+                    hl = ht[gm - along];
+                    hr = ht[gm + along];
+                }
+                for (; w; w &= w - 1) {
+                    const int t = __ffs(w) - 1;
+                    int k = c + t;
+                    if (k <= done) continue;  // already run inside a cascade
+                    const double tzv = __shfl_sync(0xffffffffu, tz, t), fsv = __shfl_sync(0xffffffffu, fs, t);
+                    double zn = __shfl_sync(0xffffffffu, zr, t), hln = __shfl_sync(0xffffffffu, hl, t),
+                           hrn = __shfl_sync(0xffffffffu, hr, t);
+                    for (;;) {
+                        done = k;
+                        const bool left = is_one(k - 1), right = is_one(k + 1);
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (left) open(k - 1, tzv, fsv, hln);
+                            if (right) open(k + 1, tzv, fsv, hrn);
                         }
+                        __syncwarp();
+                        if (!right || k + 1 > kb) break;
+                        k++;  // the opened cell now holds tzv
+                        if (!(tzv > zn)) {
+                            done = k;
+                            break;
+                        }
+                        const int gk = base + k * along;
+                        zn = z[gk + along];
+                        hln = ht[gk - along];
+                        hrn = ht[gk + along];
                     }
                 }
             }
-            __syncwarp();
+        }
+        if (opened != 0.0) atomicAdd(&g.budget[kBudOpen], opened);
+    }
+
+    // The closing pass of word q's cells, and the marks of its changed cells, by one warp;
+    // returns the depth closed by this lane.
+    __device__ __forceinline__ double close_word(const DevGrid& g, int q, unsigned wcl, unsigned wop) const {
+        const int lane = threadIdx.x & 31;
+        const int k = org + q * 32 + lane;
+        double closed = 0.0;
+        if ((wcl >> lane) & 1u) {
+            const int gp = base + k * along;
+            if (interior(g)) closed = g.H_moi[gp];
+            g.t_u[gp - g.P] = 0;
+            g.t_u[gp] = 0;
+            g.t_v[gp - 1] = 0;
+            g.t_v[gp] = 0;
+            g.khouot[gp] = 1;
+            g.colB[byte_of(g, k)] = 1;
+            g.FS[gp] = 0;
+        }
+        if (((wcl | wop) >> lane) & 1u)
+            mark_dirty(ROWS ? g.dirty_c : g.dirty_r, ROWS ? g.dlist_c : g.dlist_r, g.dctr + (ROWS ? 1 : 0), k);
+        return closed;
+    }
+
+    __device__ __forceinline__ void scan(const DevGrid& g) const {
+        warp_runs(g, wet, nq, org, lo < 2 ? 2 : lo, hi > L ? L : hi, L, ROWS ? g.daui + line * HYD_SEGL : g.dauj + line * HYD_SEGL,
+                  ROWS ? g.cuoii + line * HYD_SEGL : g.cuoij + line * HYD_SEGL, moc(g));
+    }
+};
+
+// A row by a CTA (blockDim.x a multiple of 32: each warp pass covers whole words): the mask,
+// t_z and z are staged with coalesced loads, and update_h_moi is applied here.
+__device__ __forceinline__ void reset_row_body(const DevGrid& g, const DevParams& p, int force, int bx) {
+    extern __shared__ unsigned rsm[];
+    const int line = 1 + bx;
+    const ResetLine<1> r(g, line, rsm);
+    if (r.empty()) {
+        if (force && line >= 2 && threadIdx.x == 0) *r.moc(g) = 0;
+        return;
+    }
+    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int kb0 = r.org; kb0 <= r.k1; kb0 += T) {  // uniform over the CTA
+        const int k = kb0 + tid;
+        bool c0 = false, cl = false;
+        int kv = 2;
+        if (k >= r.k0 && k <= r.k1) {
+            const int gp = r.base + k;
+            kv = g.khouot[gp];
+            const double tz = g.t_z[gp];
+            c0 = k >= 2 && k <= r.L && tz > g.z[gp];
+            if (k >= 1 && k <= r.L && kv == 0) {
+                const double hv = g.htaiz[gp] + tz;
+                g.H_moi[gp] = hv;
+                cl = k >= 2 && hv <= p.H_TINH;
+            }
+        }
+        const unsigned c0b = __ballot_sync(0xffffffffu, c0), clb = __ballot_sync(0xffffffffu, cl),
+                       oneb = __ballot_sync(0xffffffffu, kv == 1), wetb = __ballot_sync(0xffffffffu, kv == 0);
+        const int q = (kb0 - r.org + warp * 32) >> 5;
+        if (lane == 0 && kb0 + warp * 32 <= r.k1) {
+            r.c0[q] = c0b;
+            r.one[q] = oneb;
+            r.wet[q] = wetb;
+            r.cl[q] = clb;
+            r.op[q] = 0;
         }
     }
-    if (opened != 0.0) atomicAdd(&g.budget[kBudOpen], opened);
     __syncthreads();
-    // closing pass (loop 2): independent per cell
+    if (warp == 0) r.open_pass(g, p);
+    __syncthreads();
+    bool changed = false;
     double closed = 0.0;
-    for (int q = warp; q < nq; q += T >> 5) {
-        if (!((clw[q] >> lane) & 1u)) continue;
-        const int k = k0 + q * 32 + lane;
-        const int gp = base + k * along;
-        if (interior_line) closed += H[gp];
-        g.t_u[gp - P] = 0;
-        g.t_u[gp] = 0;
-        g.t_v[gp - 1] = 0;
-        g.t_v[gp] = 0;
-        kh[gp] = 1;
-        g.colB[ROWS ? (size_t)k * g.LT + line : (size_t)line * g.LT + k] = 1;
-        khs[k - k0] = 1;
-        FS[gp] = 0;
-        s_changed = 1;
-        mark_dirty(oflags, olist, octr, k);
+    for (int q = warp; q < r.nq; q += T >> 5) {
+        const unsigned wcl = r.cl[q], wop = r.op[q];
+        if (!(wcl | wop)) continue;
+        changed = true;
+        closed += r.close_word(g, q, wcl, wop);
+        if (lane == 0) r.wet[q] &= ~wcl;
     }
     if (closed != 0.0) atomicAdd(&g.budget[kBudClose], closed);
-    __syncthreads();
-    if (tid < 32 && line >= 2 && (s_changed || force))
-        warp_scan_line(g, WetShared{khs, k0}, lo, hi, L, c0w, dau, cuoi, moc);
-    __syncthreads();  // keep the other warps resident while warp 0 scans
+    if (__syncthreads_or(changed) || force) {
+        if (warp == 0 && line >= 2) r.scan(g);
+        __syncthreads();  // keep the other warps resident while warp 0 scans
+    }
 }
 
-template <int ROWS>
-__global__ void k_reset(DevGrid g, DevParams p, int force) {
-    reset_body<ROWS>(g, p, force, blockIdx.x);
+// A column by a warp, `blockDim.x / 32` columns per CTA: its column-major bytes, which the
+// preceding smoothing pass wrote (mask, t_z > z, wet with H <= H_TINH; it also applied
+// update_h_moi), are 16 cells per lane and load.  Dependent steps of a few cycles each between
+// two or three memory round trips: a CTA per column spent them on barriers, and its other
+// warps' slots on waiting (1048 x 980: 9.1 us, now 7.6; 2048 x 2048: 17.5, now 11.6; 16 reaches in
+// one launch each: a step of 360 us, now 344).
+__device__ __forceinline__ void reset_col_body(const DevGrid& g, const DevParams& p, int force, int bx) {
+    extern __shared__ unsigned rsm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int line = 1 + bx * (blockDim.x >> 5) + warp;
+    if (line > g.M) return;
+    const ResetLine<0> r(g, line, rsm + warp * kResetSets * reset_words(g.N));
+    if (r.empty()) {
+        if (force && line >= 2 && lane == 0) *r.moc(g) = 0;
+        return;
+    }
+    // a column starts on a 32-byte boundary and holds LT >= N + 3 bytes, LT a multiple of 32:
+    // the load of a lane at c <= k1 <= N + 2 ends within it
+    const unsigned char* col = g.colB + (size_t)line * g.LT;
+    constexpr int U = 2;
+    for (int b0 = r.org; b0 <= r.k1; b0 += 512 * U) {
+        uint4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int c = b0 + 512 * u + lane * 16;
+            v[u] = make_uint4(0x02020202u, 0x02020202u, 0x02020202u, 0x02020202u);
+            if (c <= r.k1) v[u] = *reinterpret_cast<const uint4*>(col + c);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int c = b0 + 512 * u + lane * 16, h = (c - r.org) >> 4;
+            if (h >= 2 * r.nq) continue;
+            const unsigned x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            // bit 0 of each byte, as 4 bits
+            auto nib = [](unsigned y) { return ((y & 0x01010101u) * 0x01020408u) >> 24; };
+            unsigned c0 = 0, one = 0, wet = 0, cl = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                one |= nib(x[i] & ~(x[i] >> 1)) << (4 * i);
+                wet |= nib(~(x[i] | (x[i] >> 1))) << (4 * i);
+                c0 |= nib(x[i] >> 2) << (4 * i);
+                cl |= nib(x[i] >> 3) << (4 * i);
+            }
+            const unsigned in = range_bits(c, r.k0, r.k1);
+            reinterpret_cast<unsigned short*>(r.c0)[h] = (unsigned short)(c0 & in);
+            reinterpret_cast<unsigned short*>(r.one)[h] = (unsigned short)(one & in);
+            reinterpret_cast<unsigned short*>(r.wet)[h] = (unsigned short)(wet & in);
+            reinterpret_cast<unsigned short*>(r.cl)[h] = (unsigned short)(cl & in);
+            reinterpret_cast<unsigned short*>(r.op)[h] = 0;
+        }
+    }
+    __syncwarp();
+    r.open_pass(g, p);
+    __syncwarp();
+    bool changed = false;
+    double closed = 0.0;
+    for (int q0 = 0; q0 < r.nq; q0 += 32) {
+        const int q = q0 + lane;
+        const unsigned wcl = q < r.nq ? r.cl[q] : 0u, wop = q < r.nq ? r.op[q] : 0u;
+        if (wcl) r.wet[q] &= ~wcl;
+        for (unsigned nz = __ballot_sync(0xffffffffu, (wcl | wop) != 0); nz; nz &= nz - 1) {
+            const int t = __ffs(nz) - 1;
+            changed = true;
+            closed += r.close_word(g, q0 + t, __shfl_sync(0xffffffffu, wcl, t), __shfl_sync(0xffffffffu, wop, t));
+        }
+    }
+    if (closed != 0.0) atomicAdd(&g.budget[kBudClose], closed);
+    __syncwarp();
+    if ((changed || force) && line >= 2) r.scan(g);
 }
-template <int ROWS>
-__global__ void k_reset_b(BatchRef br, int force) {
+
+__global__ void k_reset_rows(DevGrid g, DevParams p, int force) { reset_row_body(g, p, force, blockIdx.x); }
+__global__ void k_reset_cols(DevGrid g, DevParams p, int force) { reset_col_body(g, p, force, blockIdx.x); }
+__global__ void k_reset_rows_b(BatchRef br, int force) {
     const BatchMember bm(br);
-    reset_body<ROWS>(bm.g, bm.p, force, bm.bx);
+    reset_row_body(bm.g, bm.p, force, bm.bx);
+}
+__global__ void k_reset_cols_b(BatchRef br, int force) {
+    const BatchMember bm(br);
+    reset_col_body(bm.g, bm.p, force, bm.bx);
 }
 
 // Column-major mask bytes of the whole grid (the cells outside the extended spans keep
@@ -2411,8 +2528,8 @@ size_t scan_smem(const DevGrid& g) {
     const int L = g.N > g.M ? g.N : g.M;
     return sizeof(unsigned) * (kScanThreads / 32) * ((L + 63) / 32 + 1);
 }
-// dynamic shared memory of k_reset: the line's mask bytes and two bitsets / scan words
-size_t reset_smem(int L) { return ((L + 3 + 15) & ~15) + 3 * sizeof(unsigned) * reset_words(L); }
+// dynamic shared memory of the resets: a line's bitsets
+size_t reset_smem(int L) { return kResetSets * sizeof(unsigned) * reset_words(L); }
 int scan_grid() {
     static int nsm = 0;
     if (!nsm) {
@@ -2422,6 +2539,13 @@ int scan_grid() {
         if (nsm < 1) nsm = 1;
     }
     return nsm;
+}
+// Columns (warps) per CTA of the column resets for `cols` columns of N cells: one while the SMs
+// hold them all at once, then four; fewer where four columns' bitsets would take much of an SM.
+int reset_col_warps_of(int N, int cols) {
+    int w = cols > 4 * scan_grid() ? 4 : 1;
+    while (w > 1 && w * reset_smem(N) > 16384) w /= 2;
+    return w;
 }
 void scan_dirty(const DevGrid& g, const DevParams& p, int rows, int with_edges, cudaStream_t s) {
     const int nb = scan_grid();
@@ -2456,8 +2580,8 @@ cudaError_t grid_setup(int N, int M) {
     if ((e = allow_smem((const void*)k_explicit_v<double>, sizeof(double) * (M + 3))) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_explicit_u<float>, sizeof(double) * (N + 3))) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_explicit_v<float>, sizeof(double) * (M + 3))) != cudaSuccess) return e;
-    if ((e = allow_smem((const void*)k_reset<1>, reset_smem(M))) != cudaSuccess) return e;
-    if ((e = allow_smem((const void*)k_reset<0>, reset_smem(N))) != cudaSuccess) return e;
+    if ((e = allow_smem((const void*)k_reset_rows, reset_smem(M))) != cudaSuccess) return e;
+    if ((e = allow_smem((const void*)k_reset_cols, reset_smem(N) * reset_col_warps_of(N, M))) != cudaSuccess) return e;
     return cudaSuccess;
 }
 
@@ -2617,12 +2741,13 @@ void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, int s
 }
 
 void launch_reset_rows(const DevGrid& g, const DevParams& p, int force, int threads, cudaStream_t s) {
-    k_reset<1><<<g.N, threads, reset_smem(g.M), s>>>(g, p, force);
+    k_reset_rows<<<g.N, threads, reset_smem(g.M), s>>>(g, p, force);
     hyd_kernel_launches_add(1);
 }
 
-void launch_reset_cols(const DevGrid& g, const DevParams& p, int force, int threads, cudaStream_t s) {
-    k_reset<0><<<g.M, threads, reset_smem(g.N), s>>>(g, p, force);
+void launch_reset_cols(const DevGrid& g, const DevParams& p, int force, cudaStream_t s) {
+    const int w = reset_col_warps_of(g.N, g.M);
+    k_reset_cols<<<(g.M + w - 1) / w, 32 * w, w * reset_smem(g.N), s>>>(g, p, force);
     hyd_kernel_launches_add(1);
 }
 
@@ -2798,8 +2923,8 @@ void launch_mom_u_batch(const BatchRef& br, int ctas, int mixed, cudaStream_t s)
 }
 
 void launch_reset_batch(const BatchRef& br, int ctas, int rows, int threads, size_t smem, cudaStream_t s) {
-    if (rows) k_reset_b<1><<<ctas, threads, smem, s>>>(br, 0);
-    else k_reset_b<0><<<ctas, threads, smem, s>>>(br, 0);
+    if (rows) k_reset_rows_b<<<ctas, threads, smem, s>>>(br, 0);
+    else k_reset_cols_b<<<ctas, threads, smem, s>>>(br, 0);
     hyd_kernel_launches_add(1);
 }
 
@@ -2833,12 +2958,14 @@ cudaError_t batch_grid_setup(size_t smem_ev, size_t smem_rr, size_t smem_rc, siz
         if ((e = allow_smem(f, smem_pf)) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_explicit_v_b<double>, smem_ev)) != cudaSuccess) return e;
     if ((e = allow_smem((const void*)k_explicit_v_b<float>, smem_ev)) != cudaSuccess) return e;
-    if ((e = allow_smem((const void*)k_reset_b<1>, smem_rr)) != cudaSuccess) return e;
-    if ((e = allow_smem((const void*)k_reset_b<0>, smem_rc)) != cudaSuccess) return e;
+    if ((e = allow_smem((const void*)k_reset_rows_b, smem_rr)) != cudaSuccess) return e;
+    if ((e = allow_smem((const void*)k_reset_cols_b, smem_rc)) != cudaSuccess) return e;
     return cudaSuccess;
 }
 
-// Shared memory the batched line kernels of one grid need (k_explicit_v, k_reset rows /
+int reset_col_warps(int N, int cols) { return reset_col_warps_of(N, cols); }
+
+// Shared memory the batched line kernels of one grid need (k_explicit_v, the resets of rows /
 // columns, k_post_fused).
 void line_smem(int N, int M, size_t* ev, size_t* rr, size_t* rc, size_t* pf) {
     DevGrid g{};

@@ -186,16 +186,29 @@ __device__ __forceinline__ void BatchLines::at(int li, int& m, int& line) const 
 
 // This CTA's member, and its index bx among the member's gx CTAs (what blockIdx.x and
 // gridDim.x are in a launch for that member alone).
+// Each lane compares one start: the search is one load, where halving a list of 16 members was
+// four dependent ones at the head of every CTA.
 struct BatchMember {
     int m, bx, gx;
     const DevGrid& g;
     const DevParams& p;
     __device__ __forceinline__ explicit BatchMember(const BatchRef& br)
-        : m(batch_member_of(br.bstart, br.nm, (int)blockIdx.x)),
-          bx((int)blockIdx.x - br.bstart[m]),
-          gx(br.bstart[m + 1] - br.bstart[m]),
-          g(br.g[m]),
-          p(br.p[m]) {}
+        : m(find(br, bx)), gx(br.bstart[m + 1] - ((int)blockIdx.x - bx)), g(br.g[m]), p(br.p[m]) {}
+
+private:
+    static __device__ __forceinline__ int find(const BatchRef& br, int& bx) {
+        const int b = (int)blockIdx.x, lane = threadIdx.x & 31;
+        int m = -1, start = 0;
+        for (int k = 0; k < br.nm; k += 32) {
+            const int v = k + lane < br.nm ? br.bstart[k + lane] : 0x7fffffff;
+            const int n = __popc(__ballot_sync(0xffffffffu, v <= b));  // sorted: the first n
+            if (n == 0) break;
+            m = k + n - 1;
+            start = __shfl_sync(0xffffffffu, v, n - 1);
+        }
+        bx = b - start;
+        return m;
+    }
 };
 
 // Column-major copy k of a per-cell quantity; (row i, column j) is at [j * g.LT + i].

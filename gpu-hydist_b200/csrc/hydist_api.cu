@@ -1137,7 +1137,7 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     std::swap(g.t_v, s->scratch_v);
     if (force) launch_mark_all_cols(g, st);
     if (!fh) cudaStreamWaitEvent(st, s->ev_bjoin, 0);
-    { PHASE(PH_RESET_ROWS); launch_reset_rows(g, p, force, s->thr_r, st); }
+    { PHASE(PH_RESET_ROWS); launch_reset_rows(g, p, force, st); }
     // after a span-limited pass the update, the column rescan and (with sediment) VTH/K
     // share one launch; whole-grid passes keep them apart
     const int fuse1 = !fh && !fsd;
@@ -1848,7 +1848,7 @@ struct BatchFused {
     double* gscr = nullptr;     // sweep rows of lines too long for shared memory (if any)
     double* gscr_fs = nullptr;  // the same for the sediment sweep beside the main chain
     int thr_r = 64;
-    int rcw = 1;  // columns per CTA of the column resets
+    int rcw = 1, rrw = 1;  // columns / rows per CTA of the resets
     size_t sm_ev = 0, sm_rr = 0, sm_rc = 0, sm_pf = 0;
     cudaStream_t st = nullptr, side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
@@ -1980,13 +1980,15 @@ int fused_build(HydBatch* b) {
     std::vector<double*> outs[4];
     std::vector<int> counts[BP_COUNT];
     std::vector<int> lines[BL_COUNT], firsts[BL_COUNT];
-    int Nmax = 0, Mmax = 0, cols = 0;
+    int Nmax = 0, Mmax = 0, cols = 0, rows = 0;
     for (HydSim* s : b->members) {
         Nmax = std::max(Nmax, s->N);
         Mmax = std::max(Mmax, s->M);
         cols += s->M;
+        rows += s->N;
     }
-    f.rcw = reset_col_warps(Nmax, cols);
+    f.rcw = reset_warps(Nmax, cols);
+    f.rrw = reset_warps(Mmax, rows);
     for (HydSim* s : b->members) {
         const DevGrid g0 = s->g;
         double *A = g0.t_u, *Bu = s->scratch_u, *C = g0.t_v, *D = s->scratch_v;
@@ -2009,7 +2011,7 @@ int fused_build(HydBatch* b) {
         counts[BP_SM].push_back(rw);
         counts[BP_SM_FSB].push_back(rw + 1);
         counts[BP_EV].push_back(N - 1);
-        counts[BP_RR].push_back(N);
+        counts[BP_RR].push_back((N + f.rrw - 1) / f.rrw);
         counts[BP_RC].push_back((M + f.rcw - 1) / f.rcw);
         counts[BP_PF].push_back(row_warp_ctas(g0, N + 1) + 32 + 16);
         counts[BP_FSJC].push_back(((N - 1) * 32 + 255) / 256);
@@ -2026,7 +2028,7 @@ int fused_build(HydBatch* b) {
         size_t ev, rr, rc, pf;
         line_smem(N, M, &ev, &rr, &rc, &pf);
         f.sm_ev = std::max(f.sm_ev, ev);
-        f.sm_rr = std::max(f.sm_rr, rr);
+        f.sm_rr = std::max(f.sm_rr, f.rrw * rr);
         f.sm_rc = std::max(f.sm_rc, f.rcw * rc);
         f.sm_pf = std::max(f.sm_pf, pf);
     }
@@ -2114,7 +2116,7 @@ void fused_launch_step(HydBatch* b, int sed1, int sed2, int bed) {
     launch_smooth_batch(BR(0, BP_SM_BUD), f.ctas[BP_SM_BUD], 1, f.outs[0], 0, 0, 1, st);
     launch_explicit_v_batch(BR(1, BP_EV), f.ctas[BP_EV], f.thr_r, f.sm_ev, mx, st);
     launch_smooth_batch(BR(1, BP_SM), f.ctas[BP_SM], 0, f.outs[1], 0, 0, 0, st);
-    launch_reset_batch(BR(2, BP_RR), f.ctas[BP_RR], 1, f.thr_r, f.sm_rr, st);
+    launch_reset_batch(BR(2, BP_RR), f.ctas[BP_RR], 1, 32 * f.rrw, f.sm_rr, st);
     launch_post_fused_batch(BR(2, BP_PF), f.ctas[BP_PF], 0, sed1, mx, f.sm_pf, st);
     if (sed1) {  // the first half-step's sediment beside the second half-step (as launch_step)
         cudaEventRecord(f.fork, st);

@@ -410,7 +410,7 @@ void launch_explicit_v(const DevGrid& g, const DevParams& p, int threads, cudaSt
 void launch_explicit_u(const DevGrid& g, const DevParams& p, int threads, cudaStream_t s);
 void launch_coef_eu(const DevGrid& g, const DevParams& p, cudaStream_t s);
 // threads: a multiple of 32
-void launch_reset_rows(const DevGrid& g, const DevParams& p, int force, int threads, cudaStream_t s);
+void launch_reset_rows(const DevGrid& g, const DevParams& p, int force, cudaStream_t s);
 void launch_reset_cols(const DevGrid& g, const DevParams& p, int force, cudaStream_t s);
 void launch_spans(const DevGrid& g, cudaStream_t s);
 // n <= kPutDoubles values from host memory to dst through the launch parameters (returns
@@ -472,5 +472,5 @@ void launch_fs_sweep_batch(int dir, const BatchLines& bl, const SweepPlan& sp, i
                            double* scratch, int grid, cudaStream_t s);
 cudaError_t batch_grid_setup(size_t smem_ev, size_t smem_rr, size_t smem_rc, size_t smem_pf);
 cudaError_t batch_sweep_setup();
-int reset_col_warps(int N, int cols);
+int reset_warps(int L, int lines);
 void line_smem(int N, int M, size_t* ev, size_t* rr, size_t* rc, size_t* pf);

@@ -913,8 +913,10 @@ template <int TILE, class R>
 __global__ void __launch_bounds__(256) k_coef_fsj(DevGrid g, DevParams p, int half, int wpc) {
     coef_fsj_body<TILE, R>(g, p, half, wpc, blockIdx.x);
 }
+// Three CTAs per SM, where 89 registers allow two: the batch's 1100 CTAs are one wave less (a
+// step of 16 reaches 332 us, now 322; one reach's launch is no faster for it).
 template <int TILE, class R>
-__global__ void __launch_bounds__(256) k_coef_fsj_b(BatchRef br, int half) {
+__global__ void __launch_bounds__(256, 3) k_coef_fsj_b(BatchRef br, int half) {
     const BatchMember bm(br);
     coef_fsj_body<TILE, R>(bm.g, bm.p, half, 1, bm.bx);
 }

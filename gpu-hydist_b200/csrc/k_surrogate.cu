@@ -784,6 +784,14 @@ int sm_count() {
 }
 constexpr int kSmemMax = 232448 - 1024;  // dynamic shared memory of a CTA (227 KB less the static part)
 
+// Lets kernel f be launched with any plan's shared memory.  Always the same limit: it is the
+// context's, shared by every thread, and one lowered to a small image's plan would fail the
+// launch that another thread makes for a large one.
+template <class F>
+cudaError_t allow_smem(F* f) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+}
+
 FastDiv fast_div(uint32_t d) {
     int l = 0;
     while ((1ull << l) < d) l++;
@@ -915,8 +923,7 @@ cudaError_t launch_conv(const ConvArgs& a, cudaStream_t s) {
     const TilePlan pl = conv_plan<MODE>(a.B, a.Hin, a.Win, a.Hout, a.Wout, CIN, (size_t)(9 * CIN / 16) * NCOL * 32 + NCOL * 4,
                                         nsm, &smem);
     if (pl.T == 0) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(k_conv_tc<MODE, CIN, NCOL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem(k_conv_tc<MODE, CIN, NCOL>);
     if (e != cudaSuccess) return e;
     const int grid = (int)(pl.nstep < nsm ? pl.nstep : nsm);
     k_conv_tc<MODE, CIN, NCOL><<<grid, kConvThreads, smem, s>>>(a, pl);
@@ -958,8 +965,7 @@ cudaError_t launch_wgrad(const WgradArgs& a, cudaStream_t s) {
     size_t smem = 0;
     const TilePlan pl = wgrad_plan<MODE>(a.B, a.Hin, a.Win, a.Hout, a.Wout, CIN, &smem);
     if (pl.S == 0) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad_tc<MODE, CIN, NCOL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem(k_conv_wgrad_tc<MODE, CIN, NCOL>);
     if (e != cudaSuccess) return e;
     const int nsm = sm_count();
     const int per = (int)((pl.nstep + nsm - 1) / nsm);

@@ -1451,11 +1451,12 @@ static int residual_launch(HydSim* h, int snapshot, double** tot_out) {
     const size_t field = (size_t)(h->N + 3) * h->pitch;
     const int nb = 2 * 148;
     if (!h->res_buf) {
-        // three snapshot fields, the CTAs' sums, five results and the finished-CTA count
+        // three snapshot fields, the CTAs' sums, five results and the finished-CTA count (cleared:
+        // a snapshot leaves the cells outside the spans as they are)
         const size_t n = 3 * field + (size_t)nb * 4 + 6;
         double* p = nullptr;
         CUDA_TRY(cudaMalloc(&p, n * sizeof(double)));
-        const cudaError_t e = cudaMemsetAsync(p + n - 1, 0, sizeof(double), h->stream);
+        const cudaError_t e = cudaMemsetAsync(p, 0, n * sizeof(double), h->stream);
         if (e != cudaSuccess) cudaFree(p);
         CUDA_TRY(e);
         h->res_buf = p;

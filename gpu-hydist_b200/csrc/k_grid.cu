@@ -2444,12 +2444,13 @@ __global__ void k_add_levels_faces(DevGrid g, int i0, int j0, int rows, int cols
 
 // hyd_steady_residual: sums over the wet cells of 2..N x 2..M of (u - u0)^2 + (v - v0)^2,
 // u^2 + v^2, (z - z0)^2 and H_moi^2 into out[0..3], and the device status word into out[4];
-// with snapshot, the cell's u, v, z are copied to u0, v0, z0 after they are read.  One warp
-// per row over the row's span of cells that can be wet (4 % of a 1048 x 980 reach); each CTA's
-// sums go to part, and the last CTA to finish (counted at *count, which it resets) adds them,
-// thread by thread and then as a tree, so the order is fixed.  A cell at a time over the whole
-// grid, its row and column by 64-bit divisions, with one thread adding the CTAs' sums, made the
-// call with its synchronisation 65 us on 1048 x 980, now 37: launch, dependent loads and wait.
+// with snapshot, u, v and z of every cell that can be wet are copied to u0, v0, z0 after they are
+// read (a cell dry now may be wet when it is compared).  One warp per row over the row's span of
+// such cells (4 % of a 1048 x 980 reach); each CTA's sums go to part, and the last CTA to finish
+// (counted at *count, which it resets) adds them, thread by thread and then as a tree, so the
+// order is fixed.  A cell at a time over the whole grid, its row and column by 64-bit divisions,
+// with one thread adding the CTAs' sums, made the call with its synchronisation 65 us on
+// 1048 x 980, now 37: launch, dependent loads and wait.
 __global__ void __launch_bounds__(256) k_resid(DevGrid g, double* __restrict__ u0, double* __restrict__ v0,
                                                double* __restrict__ z0, int snapshot, double* part, unsigned* count,
                                                double* out) {
@@ -2463,16 +2464,16 @@ __global__ void __launch_bounds__(256) k_resid(DevGrid g, double* __restrict__ u
             const int gp = i * g.P + j;
             const double u = g.u[gp], v = g.v[gp], z = g.z[gp], H = g.H_moi[gp];
             const double du = u - u0[gp], dv = v - v0[gp], dz = z - z0[gp];
-            if (g.khouot[gp] != 0) continue;
-            a += du * du + dv * dv;
-            b += u * u + v * v;
-            c += dz * dz;
-            d += H * H;
             if (snapshot) {
                 u0[gp] = u;
                 v0[gp] = v;
                 z0[gp] = z;
             }
+            if (g.khouot[gp] != 0) continue;
+            a += du * du + dv * dv;
+            b += u * u + v * v;
+            c += dz * dz;
+            d += H * H;
         }
     }
     auto tree = [&]() {

@@ -166,8 +166,11 @@ struct BndSeg {
     double value, cv;
 };
 
-// Every load that does not need another's value is issued before the first test (the tables of
-// an edge without any are null): one memory round trip instead of four in a row.
+// Every load that does not need another's value is issued before the first test: one memory round
+// trip instead of four in a row.  So an edge's tables are read whether or not a segment is open
+// there: each edge has at least one row of them (zeros where the caller gave none), the host
+// refuses times past their end, and before their start (a run begun at a negative time, which
+// nothing refuses while no edge is open) they are not read.
 __device__ __forceinline__ BndSeg bnd_segment(const DevGrid& g, const EdgeArgs& a, double t) {
     BndSeg s{1, 0, 0, 0.0, 0.0};
     const int tt = g.total_time;
@@ -177,11 +180,11 @@ __device__ __forceinline__ BndSeg bnd_segment(const DevGrid& g, const EdgeArgs& 
     const int moc = a.moc[a.location], lo = a.dau[a.location * HYD_SEGL], hi = a.cuoi[a.location * HYD_SEGL],
               type = a.btype[seg_no];
     double b0 = 0.0, b1 = 0.0, c0 = 0.0, c1 = 0.0;
-    if (a.bcv) {
+    if (a.bcv && t1 >= 0) {
         b0 = a.bcv[seg_no * tt + t1];
         b1 = a.bcv[seg_no * tt + t1 + 1];
     }
-    if (a.ccv) {
+    if (a.ccv && t1 >= 0) {
         c0 = a.ccv[seg_no * tt + t1];
         c1 = a.ccv[seg_no * tt + t1 + 1];
     }

@@ -516,6 +516,78 @@ __host__ __device__ constexpr int wg_tap(int q, int h) {
     return s == 0 ? (h == 0 ? r + 1 : r + 2) : (h == 0 ? -1 : r);                     // dx 0, +1 | -1
 }
 
+// The row half that sums tap t.
+template <int MODE>
+__device__ __forceinline__ int wg_half(int t) {
+    for (int q = 0; q < 6; q++)
+        if (wg_tap<MODE>(q, 1) == t) return 1;
+    return 0;
+}
+
+// dW[n][t], all input channels, over the output pixels of raster positions p0..p1-1: each pixel's
+// dY times the input pixel of the tap, times zero where the image has none.  Only for operands
+// that are not finite (5.5 to 6.2 ms for a layer of 746k pixels of 48 channels, 0.1 ms with finite
+// operands); U pixels' loads at a time, since a thread waits for each.
+template <int MODE, int CIN, int NCOL>
+__device__ __noinline__ void wgrad_tap(const WgradArgs& a, const TilePlan& pl, long long p0, long long p1, int n, int t) {
+    constexpr int U = 2, V = CIN / 8;
+    float sum[CIN];
+#pragma unroll
+    for (int k = 0; k < CIN; k++) sum[k] = 0.0f;
+    const int dy = t / 3 - 1, dx = t % 3 - 1;
+    int b, y, x;
+    raster_at(pl, p0, b, y, x);
+    // pixel by pixel: up, a position is four output pixels
+    constexpr int per = MODE == kUp ? 4 : 1;
+    const long long count = (p1 - p0) * per;
+    int c = 0;  // which of them
+    for (long long k0 = 0; k0 < count && b < a.B; k0 += U) {
+        bool live[U];
+        __nv_bfloat16 g[U];
+        uint4 v[U][V];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int oy = MODE == kUp ? 2 * y + (c >> 1) : y, ox = MODE == kUp ? 2 * x + (c & 1) : x;
+            live[u] = b >= 0 && b < a.B && oy < a.Hout && ox < a.Wout && k0 + u < count;
+            int iy = MODE == kDown ? 2 * oy + dy : oy + dy, ix = MODE == kDown ? 2 * ox + dx : ox + dx;
+            bool in = live[u];
+            if (MODE == kUp) {
+                in = in && !((oy - dy) & 1) && !((ox - dx) & 1);
+                iy = (oy - dy) >> 1;
+                ix = (ox - dx) >> 1;
+            }
+            in = in && iy >= 0 && iy < a.Hin && ix >= 0 && ix < a.Win;
+            g[u] = a.dy[live[u] ? (((long long)b * a.Hout + oy) * a.Wout + ox) * NCOL + n : 0];
+            const uint4* px = reinterpret_cast<const uint4*>(a.x + (in ? (((long long)b * a.Hin + iy) * a.Win + ix) * CIN : 0));
+#pragma unroll
+            for (int k = 0; k < V; k++) v[u][k] = in ? px[k] : make_uint4(0, 0, 0, 0);
+            if (++c < per) continue;
+            c = 0;
+            if (++x < pl.Wp) continue;
+            x = 0;
+            if (++y < pl.Hp) continue;
+            y = 0;
+            b++;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!live[u]) continue;
+            const float f = __bfloat162float(g[u]);
+#pragma unroll
+            for (int k = 0; k < V; k++) {
+                const uint32_t w[4] = {v[u][k].x, v[u][k].y, v[u][k].z, v[u][k].w};
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    sum[8 * k + 2 * m] = fmaf(f, __uint_as_float(w[m] << 16), sum[8 * k + 2 * m]);
+                    sum[8 * k + 2 * m + 1] = fmaf(f, __uint_as_float(w[m] & 0xFFFF0000u), sum[8 * k + 2 * m + 1]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < CIN; k++) atomicAdd(a.dw + ((size_t)n * 9 + t) * CIN + k, sum[k]);
+}
+
 // Weight gradient: dW[n][t][ci] = sum_p dY[p][n] X[map(p, t)][ci].  MMAs with M = 128 rows (two
 // blocks of 64: the output channels n of two taps), N = the CIN input channels and K = 16
 // raster positions; both operands MN-major from planes of 8 channels, the taps as shifted
@@ -526,8 +598,9 @@ __host__ __device__ constexpr int wg_tap(int q, int h) {
 // What bounds it: 6 MMAs of 44 cycles (operand reads from shared memory) per 16 positions, 81
 // us for 1.49M pixels of 48 channels.  Measured there: 166 us; gathering every operand element
 // by 2-byte loads, one thread per (tap, channel), took 3.13 ms.
-// Where the output gradient is not finite at a pixel or the input next to an image's edge,
-// a tap that has no such pixel can be non-finite too (zero padding times infinity).
+// The raster's padding holds a zero output gradient beside real input pixels, so an input that is
+// not finite next to an image's edge makes taps non-finite that never meet it.  A CTA whose sums
+// are not all finite adds its output pixels one by one instead (wgrad_tap).
 template <int MODE, int CIN, int NCOL>
 __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tc(const __grid_constant__ WgradArgs a,
                                                                  const __grid_constant__ TilePlan pl,
@@ -651,7 +724,17 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tc(const __grid_co
         }
     }
     cp_async_wait_all();
-    __syncthreads();
+    const int row = (warp & 3) * 32 + lane, h = row >> 6, n = row & 63;
+    bool finite = true;
+    if (worker && n < a.nout) {
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            if (wg_tap<MODE>(((warp >> 2) * UN + u) / NB, h) < 0) continue;
+#pragma unroll
+            for (int k = 0; k < 16; k++) finite = finite && isfinite(acc[u][k]);
+        }
+    }
+    const bool pixels = __syncthreads_or(!finite);
     if (s_fail) {
         if (tid == 0) atomicExch(a.err, 1);
         if (!worker) {  // as in k_conv_tc
@@ -659,25 +742,29 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tc(const __grid_co
             for (int k = 0; k < 4; k++) mbar_wait(&m_done[k >> 1], k & 1, &never);
         }
         __syncthreads();
-    } else if (worker) {
-        const int row = (warp & 3) * 32 + lane, h = row >> 6, n = row & 63;
+    } else if (worker && pixels) {
+        for (int k = warp; k < 9 * ((a.nout + 31) / 32); k += kWgWorkers / 32) {
+            const int t = k % 9, nn = k / 9 * 32 + lane;
+            // rows 64..: one position further (fill_twice)
+            const long long p0 = pl.p_first + s0 * pl.S + (MODE == kUp ? 0 : wg_half<MODE>(t));
+            if (nn < a.nout) wgrad_tap<MODE, CIN, NCOL>(a, pl, p0, p0 + (s1 - s0) * pl.S, nn, t);
+        }
+    } else if (worker && n < a.nout) {
         const bool v4 = !(reinterpret_cast<uintptr_t>(a.dw) & 15);
-        if (n < a.nout) {
 #pragma unroll
-            for (int u = 0; u < UN; u++) {
-                const int c = (warp >> 2) * UN + u, q = c / NB;
-                const int t = wg_tap<MODE>(q, h);
-                if (t < 0) continue;
-                float* d = a.dw + ((size_t)n * 9 + t) * CIN + (c % NB) * 16;
-                if (v4) {
+        for (int u = 0; u < UN; u++) {
+            const int c = (warp >> 2) * UN + u, q = c / NB;
+            const int t = wg_tap<MODE>(q, h);
+            if (t < 0) continue;
+            float* d = a.dw + ((size_t)n * 9 + t) * CIN + (c % NB) * 16;
+            if (v4) {
 #pragma unroll
-                    for (int k = 0; k < 16; k += 4)
-                        atomicAdd(reinterpret_cast<float4*>(d + k),
-                                  make_float4(acc[u][k], acc[u][k + 1], acc[u][k + 2], acc[u][k + 3]));
-                } else {
+                for (int k = 0; k < 16; k += 4)
+                    atomicAdd(reinterpret_cast<float4*>(d + k),
+                              make_float4(acc[u][k], acc[u][k + 1], acc[u][k + 2], acc[u][k + 3]));
+            } else {
 #pragma unroll
-                    for (int k = 0; k < 16; k++) atomicAdd(d + k, acc[u][k]);
-                }
+                for (int k = 0; k < 16; k++) atomicAdd(d + k, acc[u][k]);
             }
         }
     }

@@ -475,7 +475,9 @@ int hyd_get_sweep_shape(hyd_handle h, int* ctas, int* wide);
  *   n < nout, c < cin, zero up to ncol and cinp (multiples of 16, at most 256); strides, so that
  *   a data gradient's channel-transposed weights are packed from the layer's own.
  * hyd_conv_wgrad: dw[n][t][c] += sum_p dy[p][n] x[map(p,t)][c] (FP32, n < nout), dy with
- *   ncol channels per pixel; map is the layer's forward mapping.
+ *   ncol channels per pixel; map is the layer's forward mapping, x zero outside the image (so
+ *   a dy that is not finite reaches every tap, an x only the taps that meet it; such operands
+ *   take a slower form).
  * hyd_bias_grad: db[n] += sum_p dy[p][n].
  * hyd_mse_grad: loss += scale sum_p w[p] |pred[p] - target[p]|^2 over nc channels (FP32),
  *   dy[p][c] = 2 scale w[p] (pred - target) as BF16 with ncol channels (zero beyond nc).

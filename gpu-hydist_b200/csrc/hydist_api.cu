@@ -73,6 +73,7 @@ struct HydSim {
     double* fs_scratch;     // the same for the sediment sweeps (which may run beside the others)
     SweepPlan plan;         // launch shapes of the sweeps
     int plan_grid;          // the sweeps' CTAs as planned at creation (the most allowed)
+    int shared;             // a batch member: other reaches' work fills the device beside its launches
     void* arena;
     size_t arena_bytes;
     std::vector<void*> extra;
@@ -553,6 +554,7 @@ int hyd_create(const HydCaseParams* p, int N, int M, int device, hyd_handle* out
     s->pitch = ((M + 3) + 31) / 32 * 32;
     s->device = device;
     s->t = 0;
+    s->shared = 0;
     s->have_boundary = 0;
     s->initialized = 0;
     const char* sv = getenv("HYD_SOLVER");
@@ -1108,7 +1110,7 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
         start_idx = 3;
         end_idx = s->M - 1;
     }
-    { PHASE(PH_COEF_UZ); launch_coef_bnd(g, p, 0, 3, s->plan.wide, st); }
+    { PHASE(PH_COEF_UZ); launch_coef_bnd(g, p, 0, 3, s->shared, st); }
     { PHASE(PH_SWEEP_UZ); launch_sweep_uz(g, p, s->plan, start_idx, end_idx, s->solver, s->sweep_scratch, st); }
     // span-limited passes: the half-step's water budget beside the smoothing and explicit v
     // (joined before the row resets change the mask); whole-grid passes keep it in the
@@ -1124,10 +1126,10 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     // owes a rescan of every line (tables set by the caller) or whole-grid passes takes it from
     // the tables, line by line, and so does v on larger grids, where its rows are contiguous
     // and a CTA per row is the faster form (4096 x 2048: 30 against 38 us)
-    const int mom = !fh && !force, msm = mom && !s->plan.wide && mom_smooths(g);
+    const int mom = !fh && !force, msm = mom && !s->shared && mom_smooths(g);
     if (msm) {
         PHASE(PH_EXPL_V);
-        launch_mom(g, p, 1, 1, s->plan.wide, s->scratch_u, st);
+        launch_mom(g, p, 1, 1, s->shared, s->scratch_u, st);
         std::swap(g.t_u, s->scratch_u);
     } else {
         { PHASE(PH_SMOOTH); launch_smooth(g, p, 1, s->scratch_u, fh, 0, 0, fh, st); }
@@ -1160,18 +1162,18 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     if (overlap) {
         cudaEventRecord(s->ev_fork, st);
         cudaStreamWaitEvent(s->side, s->ev_fork, 0);
-        { PHASE_ON(PH_COEF_FSJ, s->side); launch_coef_fsj(g, p, 0, s->plan.wide, s->side); }
+        { PHASE_ON(PH_COEF_FSJ, s->side); launch_coef_fsj(g, p, 0, s->shared, s->side); }
         { PHASE_ON(PH_FS_J, s->side); launch_fs_sweep_j(g, p, s->plan, 0, s->solver, s->fs_scratch, s->side); }
         { PHASE_ON(PH_UPDATE_FS, s->side); launch_update_fs(g, fsd, s->side); }
         cudaEventRecord(s->ev_join, s->side);
     } else if (sed1) {
         if (!(sed1 && fuse1)) { PHASE(PH_VTH); launch_vth_hesok(g, p, fsd, 0, st); }
-        { PHASE(PH_COEF_FSJ); launch_coef_fsj(g, p, 0, s->plan.wide, st); }
+        { PHASE(PH_COEF_FSJ); launch_coef_fsj(g, p, 0, s->shared, st); }
         { PHASE(PH_FS_J); launch_fs_sweep_j(g, p, s->plan, 0, s->solver, s->fs_scratch, st); }
         { PHASE(PH_UPDATE_FS); launch_update_fs(g, fsd, st); }
     }
     // ---- half-step 2: implicit along j (rows), explicit u
-    { PHASE(PH_BOUNDARY); launch_coef_bnd(g, p, 1, overlap ? 1 : 3, s->plan.wide, st); }
+    { PHASE(PH_BOUNDARY); launch_coef_bnd(g, p, 1, overlap ? 1 : 3, s->shared, st); }
     start_idx = 2;
     end_idx = s->N;
     if (p.channel && s->P.kenhhepng == 1) {
@@ -1192,7 +1194,7 @@ static void launch_step(HydSim* s, int sed1, int sed2, int bed, int force = 0, i
     }
     if (mom) {
         PHASE(PH_EXPL_U);
-        launch_mom(g, p, 0, msm, s->plan.wide, s->scratch_v, st);
+        launch_mom(g, p, 0, msm, s->shared, s->scratch_v, st);
         if (msm) std::swap(g.t_v, s->scratch_v);
     } else {
         { PHASE(PH_COEF_EU); launch_coef_eu(g, p, st); }
@@ -1899,6 +1901,7 @@ int hyd_batch_create(int count, const HydCaseParams* params, const int* dims, in
             delete b;
             return fail(rc, msg);
         }
+        h->shared = 1;
         b->members.push_back(h);
     }
     // the members run side by side: sweeps sized by the batch's lines, not the device

@@ -24,7 +24,9 @@ import math
 import time
 
 FUSED = ("fused",)
-DEFAULT_CANDIDATES = ((16, 1), (8, 1), (32, 1), (16, 0), FUSED)
+# The shapes a batch may start with, d = 16 k for k = 1 to 4 (hyd_set_sweep_shape), are among
+# them: tuning never leaves it on a slower one than it had for want of trying that.
+DEFAULT_CANDIDATES = ((16, 1), (32, 1), (48, 1), (64, 1), (8, 1), (16, 0), FUSED)
 
 
 def apply_policy(batch, policy):

@@ -406,10 +406,10 @@ void launch_widen_spans(const DevGrid& g, cudaStream_t s);
 // the smoothing of the other, swept component into out (else it is smoothed already).
 int mom_smooths(const DevGrid& g);
 void launch_mom(const DevGrid& g, const DevParams& p, int dir, int smooth, int shared, double* out, cudaStream_t s);
+// threads: a multiple of 32
 void launch_explicit_v(const DevGrid& g, const DevParams& p, int threads, cudaStream_t s);
 void launch_explicit_u(const DevGrid& g, const DevParams& p, int threads, cudaStream_t s);
 void launch_coef_eu(const DevGrid& g, const DevParams& p, cudaStream_t s);
-// threads: a multiple of 32
 void launch_reset_rows(const DevGrid& g, const DevParams& p, int force, cudaStream_t s);
 void launch_reset_cols(const DevGrid& g, const DevParams& p, int force, cudaStream_t s);
 void launch_spans(const DevGrid& g, cudaStream_t s);

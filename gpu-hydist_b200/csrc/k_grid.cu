@@ -241,8 +241,8 @@ __device__ void bnd_apply(const DevGrid& g, const EdgeArgs& a, const BndRec& r, 
 // Update_Boundary_Value (support_funcs.cu:622-668).  The reference applies the edges in
 // the order up, down, left, right (the order a converged warp applies them); two edges
 // only meet at the corner indices (2 and N of the up/down edges, 2 and M of left/right).
-// Here the four edges run at once, each in a quarter of the CTA (blockDim a multiple of
-// 128), holding back their corner writes; thread 0 then applies those in the reference's
+// Here the four edges run at once, each in a quarter of the CTA (64, 128 or 256 threads),
+// holding back their corner writes; thread 0 then applies those in the reference's
 // order, and again the (N, 2) write of the down edge and, when N > M, the (N, M) write of
 // the up edge, which threads past the first warp repeat in the reference.  `writes`
 // selects the arrays written (the same order applies within each array), so the
@@ -448,18 +448,17 @@ __device__ __forceinline__ void vz_cell_coeffs(const DevGrid& g, const DevParams
 
 // The first launch of each half-step.  KIND 0 (half-step 1): UZ coefficients of every wet
 // interior cell written column-major (g.colT arrays 0..6: a2 c2 d2 f1 f2 f3 f5), and in
-// the last CTA the clock advance and the boundary values of the half-step.  KIND 1
-// (half-step 2): VZ coefficients written row-major (g.rowC arrays 0..6), and in the last
-// CTA the half-step's boundary values (`writes`).  The coefficients read none of what the
-// boundary writes (edge levels, edge velocity arrays, inflow concentrations).  One warp
-// per row of the grid over the row's span of cells that can be wet; small CTAs, so that
-// the stores spread over many SMs; TILE (large grids, g.tile_cols) stores KIND 0 through a
+// CTA 0 the clock advance and the boundary values of the half-step.  KIND 1
+// (half-step 2): VZ coefficients written row-major (g.rowC arrays 0..6), and in CTA 0 the
+// half-step's boundary values (`writes`).  The coefficients read none of what the
+// boundary writes (edge levels, edge velocity arrays, inflow concentrations).  wpc warps
+// per row of the grid (coef_shape) over the row's span of cells that can be wet; small CTAs, so
+// that the stores spread over many SMs; TILE (large grids, g.tile_cols) stores KIND 0 through a
 // shared-memory tile (colmajor_tile), 8 rows of a column at a time.  The variants are
 // separate kernels: the tile's shared memory would otherwise shrink the L1 share of the
 // small grids' launches, whose stencil loads it serves.
-// bx, gx: the CTA's index among the launch's CTAs of this grid and their count (blockIdx.x
-// and gridDim.x of a launch for one grid; a member's share of a batched launch).
-// wpc: warps per row of the untiled form.
+// bx: the CTA's index among the launch's CTAs of this grid (blockIdx.x of a launch for one grid;
+// a member's share of a batched launch).
 template <int KIND, int TILE, class R>
 __device__ __forceinline__ void coef_bnd_body(const DevGrid& g, const DevParams& p, int writes, int wpc, int bx) {
     // CTA 0 takes the clock and the boundary (a chain of dependent loads, started first

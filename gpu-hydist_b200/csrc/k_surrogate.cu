@@ -596,7 +596,7 @@ __device__ __noinline__ void wgrad_tap(const WgradArgs& a, const TilePlan& pl, l
 // kWgChain positions into registers, so a chain of FP32 additions in it is no longer than
 // 128 MMAs, and the registers are added to dw once, with vector atomics.
 // What bounds it: 6 MMAs of 44 cycles (operand reads from shared memory) per 16 positions, 81
-// us for 1.49M pixels of 48 channels.  Measured there: 166 us; gathering every operand element
+// us for 1.49M pixels of 48 channels.  Measured there: 171 us; gathering every operand element
 // by 2-byte loads, one thread per (tap, channel), took 3.13 ms.
 // The raster's padding holds a zero output gradient beside real input pixels, so an input that is
 // not finite next to an image's edge makes taps non-finite that never meet it.  A CTA whose sums

@@ -340,7 +340,8 @@ int hyd_set_state(hyd_handle h, const void* buf, size_t bytes);
  * sediment, bed-update and hourly table schedules) to t without touching any field.
  *
  * hyd_steady_residual(h, snapshot, out, n >= 2) compares the state with the snapshot
- * taken at the previous call with snapshot = 1, over the wet cells of [2,N] x [2,M]:
+ * taken at the previous call with snapshot = 1 (of every cell that can be wet), over the
+ * cells of [2,N] x [2,M] wet now:
  *   out[0] = ||(u, v) - (u0, v0)||_2 / ||(u, v)||_2   (momentum: relative velocity change)
  *   out[1] = ||z - z0||_2 / ||H_moi||_2               (continuity: level change / depth)
  * each an FP64 sum added in a fixed order; HUGE_VAL before the first snapshot, with no
